@@ -27,6 +27,7 @@
 
 #include "apply_modal.cuh"
 #include "internal.h"
+#include "pcg_chip.h"
 
 namespace gbs {
 
@@ -1097,11 +1098,45 @@ static int pcg_fresh_setup(const gbsimp_ctx *ctx, int nx, int ny, int nz, const 
 }
 
 // Optional profiling (prof != nullptr): CUDA events around every K1 launch; only the
-// launches of iterations that actually ran (the device counter advanced) are summed.
+// launches of iterations that actually ran (the device counter advanced) are summed. The on-chip
+// form runs all iterations in one launch: events around it, counted as its iterations.
 struct ApplyProfile {
     double seconds = 0.0;
     int launches = 0;
 };
+
+// ---- the on-chip form (pcg_chip.cu) ---------------------------------------------------------
+// Whenever the grid fits the chip: it is the faster form at every size that does. us per iteration of
+// a solve, streaming in the graph loop -> on the chip: 8x4x4 7.5 -> 2.1, 32x8x8 7.9 -> 4.1, 32^3
+// 8.4 -> 4.4, 48^3 10.7 -> 5.6, 95x47x33 11.9 -> 6.7, 64^3 (about the most it holds) 13.9 -> 10.1.
+static inline bool chip_ok(const gbsimp_ctx *ctx, const ChipItem &it) {
+    return use_modal(ctx, it.nz) && chip_min_blocks(ctx, it) > 0;
+}
+
+// The workspace of the on-chip form. A paused solve's state sits in r, ap (w), p1 (s), p0 (p) and
+// the caller's u; the packets in the vectors after them (r1 .. w2 and the partial sums, all
+// unused by this form), or in `xch` when the caller has a larger idle buffer.
+static ChipItem chip_item(int nx, int ny, int nz, const PcgWs &w, float *u, void *xch = nullptr, size_t xch_bytes = 0) {
+    ChipItem it{};
+    it.nx = nx;
+    it.ny = ny;
+    it.nz = nz;
+    it.E = w.E;
+    it.dinv = w.dinv;
+    it.u = u;
+    it.sc = w.sc;
+    it.r = w.r;
+    it.w = w.ap;
+    it.s = w.p1;
+    it.p = w.p0;
+    it.xch = (float4 *)w.r1;
+    it.xch_bytes = (size_t)((char *)(w.partials + w.partial_count) - (char *)w.r1);
+    if (xch_bytes > it.xch_bytes) {
+        it.xch = (float4 *)xch;
+        it.xch_bytes = xch_bytes;
+    }
+    return it;
+}
 
 // FP32 PCG. u: x0 in, solution out. Returns GBS_OK and fills *out (status inside).
 // With out == nullptr (and no profiling) the solve is only enqueued: the device-driven paths
@@ -1110,10 +1145,49 @@ struct ApplyProfile {
 int pcg_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *glaw, const float *x, const float *b,
             const uint8_t *mask, float *u, double rtol, int max_iter, int check_every, void *ws, PcgScalars *out,
             cudaStream_t st, ApplyProfile *prof = nullptr, int fused = 0, unsigned setup_flags = 0,
-            const float2 *bdd = nullptr, const double *bscale = nullptr, bool *finish_left = nullptr) {
+            const float2 *bdd = nullptr, const double *bscale = nullptr, bool *finish_left = nullptr,
+            void *scratch = nullptr, size_t scratch_bytes = 0) {
     const int64_t nd = n_dof_of(nx, ny, nz);
     PcgWs w = pcg_ws(ws, nx, ny, nz);
     const Law<float> law = make_law<float>(*glaw);
+    {
+        ChipItem ci = chip_item(nx, ny, nz, w, u, scratch, scratch_bytes);
+        if (chip_ok(ctx, ci)) {
+            ci.fresh = (setup_flags & SETUP_X0_ZERO) && max_iter > 0;
+            ci.b = b;
+            ci.bdd = bdd;
+            ci.bscale = bscale;
+            ci.tol = rtol;
+            ci.max_iter = max_iter;
+            int rc = GBS_OK;
+            if (!ci.fresh)
+                rc = pcg_setup(ctx, nx, ny, nz, glaw, x, b, mask, u, rtol, max_iter, w, st, setup_flags);
+            else if (!(setup_flags & SETUP_KEEP_DINV))
+                rc = setup_diag(ctx, nx, ny, nz, law, x, mask, w, st);
+            if (rc) return rc;
+            cudaEvent_t ev[2] = {};
+            if (prof) {
+                for (auto &e : ev) GBS_CUDA_TRY(cudaEventCreate(&e));
+                GBS_CUDA_TRY(cudaEventRecord(ev[0], st));
+            }
+            rc = chip_run(ctx, &ci, 1, 0, st);
+            if (rc) return rc;
+            if (prof) GBS_CUDA_TRY(cudaEventRecord(ev[1], st));
+            if (!out && !prof) return GBS_OK;
+            PcgScalars h;
+            rc = read_scalars(w.sc, &h, st);
+            if (rc) return rc;
+            if (prof) {
+                float ms = 0.0f;
+                GBS_CUDA_TRY(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+                prof->seconds += 1e-3 * ms;
+                prof->launches += h.iter;
+                for (auto &e : ev) cudaEventDestroy(e);
+            }
+            if (out) *out = h;
+            return GBS_OK;
+        }
+    }
     // from x0 = 0 the one-kernel form starts with a start pass instead of the setup's apply
     // (the persistent kernel keeps the setup: it reads the scalars of iteration 0); only this
     // start takes the right-hand side as scaled (h, l) pairs
@@ -1569,6 +1643,9 @@ int solve_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *l
     const PcgScalars *pending = nullptr;
     const PcgWs pw = pcg_ws(w.pcg, nx, ny, nz);
     const bool dd = use_dd_residual(ctx, o);
+    // the residual's element buffer is idle during the inner solves: room for the exchange packets
+    const size_t scratch = apply_f64_modal_ws_bytes(nx, ny, nz);
+    const bool chip = chip_ok(ctx, chip_item(nx, ny, nz, pw, w.d32, w.elem, scratch));
     {
         int rc = outer_start(ctx, nd, u, f, mask, dd, w, st);
         if (rc) return rc;
@@ -1613,7 +1690,8 @@ int solve_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *l
         // the first round computes 1/diag, later rounds reuse it
         const unsigned flags = SETUP_X0_ZERO | (outer > 1 ? SETUP_KEEP_DINV : 0u);
         // the fresh start forms b = r / ||r|| itself from the double-float residual
-        const bool scaled_in_start = dd && fresh_start_ok(ctx, nz, o->fused, o->max_iter - total, flags);
+        const bool scaled_in_start =
+            dd && o->max_iter > total && (chip || fresh_start_ok(ctx, nz, o->fused, o->max_iter - total, flags));
         if (!scaled_in_start) {
             rc = outer_scale(ctx, nd, dd, w, st);
             if (rc) return rc;
@@ -1629,7 +1707,7 @@ int solve_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *l
             rc = pcg_run(ctx, nx, ny, nz, law, x, w.b32, mask, w.d32, itol, o->max_iter - total, o->check_every, w.pcg,
                          async ? nullptr : &ps, st, o->profile ? &prof : nullptr, o->fused, flags,
                          scaled_in_start ? (const float2 *)w.r64 : nullptr, scaled_in_start ? &w.os->scale : nullptr,
-                         dd ? &finish_left : nullptr);
+                         dd ? &finish_left : nullptr, w.elem, scratch);
         }
         if (rc) return rc;
         if (async) {
@@ -1885,6 +1963,24 @@ extern "C" int gbsimp_time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, co
         freeze_scalars_kernel<<<1, 1, 0, st>>>(w.sc);
     }
     GBS_LAUNCH_CHECK("time_pcg_apply setup");
+    const ChipItem ci = chip_item(nx, ny, nz, w, xu);
+    if (chip_ok(ctx, ci)) {  // `reps` iterations of the on-chip form, its loads and stores included
+        cudaEvent_t e0, e1;
+        GBS_CUDA_TRY(cudaEventCreate(&e0));
+        GBS_CUDA_TRY(cudaEventCreate(&e1));
+        float ms = 0.0f;
+        int rc = chip_run(ctx, &ci, 1, reps, st);  // warm-up
+        cudaError_t e = cudaSuccess;
+        if (!rc && (e = cudaEventRecord(e0, st)) == cudaSuccess && !(rc = chip_run(ctx, &ci, 1, reps, st)) &&
+            (e = cudaEventRecord(e1, st)) == cudaSuccess && (e = cudaEventSynchronize(e1)) == cudaSuccess)
+            e = cudaEventElapsedTime(&ms, e0, e1);
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        if (rc) return rc;
+        if (e != cudaSuccess) return cuda_error(e, "time_pcg_apply on-chip run");
+        *seconds_per_launch = 1e-3 * ms / reps;
+        return GBS_OK;
+    }
     if (modal) {
         const int r = modal_prepare<MODE_CG>(ctx, nz);
         if (r < 0) return -r;
@@ -2063,6 +2159,40 @@ extern "C" int gbsimp_pcg_csr_f32(gbsimp_ctx *ctx, int64_t n, const int32_t *row
 // ---- batched rounds ------------------------------------------------------------------------
 namespace gbs {
 
+// Packs on-chip solves into launches of at most `group` designs that are resident together, in
+// as few launches as first-fit finds, the load spread evenly over them. Indices into `items`.
+static std::vector<std::vector<int>> chip_groups(const gbsimp_ctx *ctx, const std::vector<ChipItem> &items, int group) {
+    std::vector<int> need(items.size()), by_size;
+    for (size_t i = 0; i < items.size(); ++i) {
+        need[i] = chip_min_blocks(ctx, items[i]);
+        by_size.push_back((int)i);
+    }
+    std::stable_sort(by_size.begin(), by_size.end(), [&](int a, int b) { return need[a] > need[b]; });
+    std::vector<std::vector<int>> out, even;
+    std::vector<int> used;
+    for (int i : by_size) {
+        size_t k = 0;
+        while (k < out.size() && (used[k] + need[i] > ctx->num_sms || (int)out[k].size() >= group)) ++k;
+        if (k == out.size()) {
+            out.emplace_back();
+            used.push_back(0);
+        }
+        out[k].push_back(i);
+        used[k] += need[i];
+    }
+    even.resize(out.size());
+    std::fill(used.begin(), used.end(), 0);
+    for (int i : by_size) {
+        size_t k = 0;
+        for (size_t j = 1; j < even.size(); ++j)
+            if (used[j] < used[k]) k = j;
+        if (used[k] + need[i] > ctx->num_sms || (int)even[k].size() >= group) return out;
+        even[k].push_back(i);
+        used[k] += need[i];
+    }
+    return even;
+}
+
 static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int n, const gbsimp_law *glaw,
                             const gbsimp_solve_opts *o, cudaStream_t st) {
     const Law<float> law = make_law<float>(*glaw);
@@ -2129,6 +2259,51 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
     std::vector<int> fresh;
     for (int i : res)
         if (items[i].state == 0) fresh.push_back(i);
+    // Grids that fit the chip run in the on-chip form, started or resumed; the others as below.
+    auto citem = [&](int i) {
+        gbsimp_batch_item &it = items[i];
+        SolveWs w = solve_ws(it.ws, it.nx, it.ny, it.nz);
+        return chip_item(it.nx, it.ny, it.nz, pcg_ws(w.pcg, it.nx, it.ny, it.nz), w.d32, w.elem,
+                         apply_f64_modal_ws_bytes(it.nx, it.ny, it.nz));
+    };
+    std::vector<int> chip_items;
+    std::vector<ChipItem> chip_started;
+    for (int i : act)
+        if (items[i].state == 0 && items[i].stats.inner_active == 1 && chip_ok(ctx, citem(i))) {
+            chip_items.push_back(i);
+            chip_started.push_back(citem(i));
+        }
+    {
+        std::vector<int> other;
+        for (int i : fresh) {
+            gbsimp_batch_item &it = items[i];
+            ChipItem ci = citem(i);
+            if (o->max_iter <= it.stats.iterations || !chip_ok(ctx, ci)) {
+                other.push_back(i);
+                continue;
+            }
+            const int64_t nd = n_dof_of(it.nx, it.ny, it.nz);
+            SolveWs w = solve_ws(it.ws, it.nx, it.ny, it.nz);
+            PcgWs pw = pcg_ws(w.pcg, it.nx, it.ny, it.nz);
+            int rc = it.stats.outer > 1 ? GBS_OK : setup_diag(ctx, it.nx, it.ny, it.nz, law, it.x, it.node_mask, pw, st);
+            if (!rc && !dd) rc = outer_scale(ctx, nd, dd, w, st);
+            if (rc) return rc;
+            double itol = o->rtol / it.stats.relres;
+            if (itol < inner) itol = inner;
+            ci.fresh = 1;
+            if (dd) {
+                ci.bdd = (const float2 *)w.r64;
+                ci.bscale = &w.os->scale;
+            } else {
+                ci.b = w.b32;
+            }
+            ci.tol = itol;
+            ci.max_iter = o->max_iter - it.stats.iterations;
+            chip_items.push_back(i);
+            chip_started.push_back(ci);
+        }
+        fresh.swap(other);
+    }
     for (int i : fresh) {
         gbsimp_batch_item &it = items[i];
         const int64_t nd = n_dof_of(it.nx, it.ny, it.nz);
@@ -2161,8 +2336,16 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
         return fused_plan(ctx, fi, (int)c.size(), &P, share) == GBS_OK;
     };
     std::vector<int> order, graph_items;
+    std::vector<char> on_chip(n, 0);
+    for (int i : chip_items) on_chip[i] = 1;
+    for (const std::vector<int> &c : chip_groups(ctx, chip_started, o->fused ? std::min(group, kChipMaxDesigns) : 1)) {
+        std::vector<ChipItem> ci;
+        for (int j : c) ci.push_back(chip_started[j]);
+        const int rc = chip_run(ctx, ci.data(), (int)ci.size(), budget, st);
+        if (rc) return rc;
+    }
     for (int i : act)
-        if (items[i].state == 0 && items[i].stats.inner_active == 1) order.push_back(i);
+        if (items[i].state == 0 && items[i].stats.inner_active == 1 && !on_chip[i]) order.push_back(i);
     for (int i : act)
         if (items[i].state == 0 && items[i].stats.inner_active == 2) graph_items.push_back(i);
     for (int i : fresh) {
@@ -2217,10 +2400,11 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
         rc = cg_publish(ctx, it.nx, it.ny, it.nz, pw, 1, st);
         if (rc) return rc;
     }
-    std::vector<int> inn(fused_items);
+    std::vector<int> inn(chip_items);
+    inn.insert(inn.end(), fused_items.begin(), fused_items.end());
     inn.insert(inn.end(), graph_items.begin(), graph_items.end());
     if (inn.empty()) return GBS_OK;
-    const size_t n_fused = fused_items.size();
+    const size_t n_fused = chip_items.size() + fused_items.size();
     // finalize the solves that ended (a paused one is left as it is), read every item's PCG
     // scalars (one sync), correct u of the ended ones
     const size_t ps = sizeof(PcgScalars);
@@ -2231,11 +2415,13 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
             const int64_t nd = n_dof_of(it.nx, it.ny, it.nz);
             SolveWs w = solve_ws(it.ws, it.nx, it.ny, it.nz);
             PcgWs pw = pcg_ws(w.pcg, it.nx, it.ny, it.nz);
-            // one-kernel graph loop: x may owe a half step; persistent: complete
+            // one-kernel graph loop: x may owe a half step; persistent, on-chip: complete
             const bool graph_loop = k + j >= n_fused;
-            pcg_finalize_kernel<<<ew_blocks(ctx, nd), 256, 0, st>>>(nd, pw.p0, pw.p1, w.d32, pw.sc,
-                                                                    use_modal(ctx, it.nz) ? (graph_loop ? 2 : 0) : 1);
-            GBS_LAUNCH_CHECK("pcg_finalize_kernel");
+            if (!on_chip[inn[k + j]]) {
+                pcg_finalize_kernel<<<ew_blocks(ctx, nd), 256, 0, st>>>(nd, pw.p0, pw.p1, w.d32, pw.sc,
+                                                                        use_modal(ctx, it.nz) ? (graph_loop ? 2 : 0) : 1);
+                GBS_LAUNCH_CHECK("pcg_finalize_kernel");
+            }
             GBS_CUDA_TRY(cudaMemcpyAsync((char *)hp + j * ps, pw.sc, ps, cudaMemcpyDeviceToHost, st));
         }
         GBS_CUDA_TRY(cudaStreamSynchronize(st));

@@ -80,7 +80,8 @@ typedef struct gbsimp_solve_opts {
                              graph-loop trips of 12 there), after which the round returns and the
                              paused solves resume in the next one; 0 = every inner PCG runs to
                              its tolerance within the round */
-    int32_t fused;        /* 1 = persistent fused PCG kernel, 0 = graph loop, one launch per iteration */
+    int32_t fused;        /* grids that the chip does not hold: 1 = persistent fused PCG kernel, 0 = graph
+                             loop, one launch per iteration */
     int32_t profile;      /* 1 = time every PCG apply launch with CUDA events (stats) */
     int32_t batch_share;  /* batched persistent launches: how the SMs are shared among the designs
                              of one launch. 0 = in proportion to element counts; 1 = in proportion
@@ -230,8 +231,9 @@ int gbsimp_pcg_f32(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *la
  * stages s, r and u = M r, applies K to u, updates p and the iterate and sums r.u, w.u and
  * r.r; dense element: the apply fused with p = z + beta p, the iterate update and p.Ap),
  * with frozen scalars. reps back-to-back launches replayed from one CUDA graph, timed with
- * CUDA events on the stream; writes the mean device time per launch. Synchronises the
- * stream. */
+ * CUDA events on the stream; writes the mean device time per launch. A grid that the chip
+ * holds runs all its iterations in one launch: reps of them, the launch's loads and stores
+ * included, and the mean per iteration. Synchronises the stream. */
 size_t gbsimp_time_pcg_apply_ws_bytes(int nx, int ny, int nz);
 int gbsimp_time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *law,
                           const float *x, const uint8_t *node_mask, int reps, void *ws,
@@ -272,7 +274,8 @@ typedef struct gbsimp_batch_item {
 
 /* One round of the FP64 defect correction for every active item: FP64 residuals (one sync
  * for all), then the FP32 PCG of every item still above rtol, then the FP64 corrections.
- * With opts->fused the PCGs run as cooperative launches of a persistent kernel, up to 24
+ * Items whose grids the chip holds run there, up to 16 designs per launch with opts->fused.
+ * Of the others, with opts->fused the PCGs run as cooperative launches of a persistent kernel, up to 24
  * items per launch (packed greedily from the items that are resident together), each item on
  * its own share of the SMs with its own grid barrier and scalars, converging independently.
  * An item that fits no such launch, or any item when opts->fused is 0, runs its own
