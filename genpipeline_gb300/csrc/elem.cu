@@ -173,10 +173,8 @@ constexpr int kMaxStencil = 1024;
 struct Stencil {
     int n;
     int r;
-    int flat;              // 1: doff[] holds the flat offsets of this grid
     int off[kMaxStencil];  // dx, dy, dz packed as signed bytes
     float w[kMaxStencil];  // rmin - dist > 0
-    int doff[kMaxStencil]; // (dx ny + dy) nz + dz: the element offset in x-y-z order
 };
 
 // The neighbourhood of simp_solver.py:1553-1565: offsets of the box of half-width
@@ -186,7 +184,6 @@ static int make_stencil(double rmin, Stencil *s) {
     const int r = (int)ceil(rmin);
     s->n = 0;
     s->r = r;
-    s->flat = 0;
     for (int di = -r; di <= r; ++di)
         for (int dj = -r; dj <= r; ++dj)
             for (int dk = -r; dk <= r; ++dk) {
@@ -203,83 +200,155 @@ static int make_stencil(double rmin, Stencil *s) {
     return GBS_OK;
 }
 
-// The flat element offsets of the stencil for a grid of ny x nz element rows, when every
-// one fits in an int (s->flat = 1; otherwise the kernel uses the bounds-checked path only).
-static void set_flat_offsets(int ny, int nz, Stencil *s) {
-    const int64_t reach = (int64_t)s->r * ((int64_t)ny * nz + nz + 1);
-    s->flat = reach < INT32_MAX ? 1 : 0;
-    if (!s->flat) return;
-    for (int q = 0; q < s->n; ++q) {
-        const int o = s->off[q];
-        const int di = (int)(int8_t)(o & 0xff), dj = (int)(int8_t)((o >> 8) & 0xff), dk = (int)(int8_t)((o >> 16) & 0xff);
-        s->doff[q] = (int)(((int64_t)di * ny + dj) * nz + dk);
-    }
-}
-
-__device__ __forceinline__ void neumaier_add(float &s, float &c, float v) {
-    const float t = s + v;
-    c += fabsf(s) >= fabsf(v) ? (s - t) + v : (v - t) + s;
-    s = t;
-}
-
 __device__ __forceinline__ void unpack_off(int o, int &di, int &dj, int &dk) {
     di = (int)(int8_t)(o & 0xff);
     dj = (int)(int8_t)((o >> 8) & 0xff);
     dk = (int)(int8_t)((o >> 16) & 0xff);
 }
 
+// The stencil as columns along z, sorted by their half-extent h: weights w[0..h] of |dz|.
+constexpr int kFilterR = 5;  // rmin <= 6, and a weight at distance 6 is zero
+constexpr int kFilterCols = (2 * kFilterR + 1) * (2 * kFilterR + 1);
+struct FilterCols {
+    int start[kFilterR + 2];  // columns of half-extent h: start[h] .. start[h + 1] - 1
+    short di[kFilterCols], dj[kFilterCols];
+    float w[kFilterCols][kFilterR + 1];
+};
+static int filter_columns(const Stencil &st, FilterCols *F) {
+    int half[2 * kFilterR + 1][2 * kFilterR + 1], R = 0, n = 0;
+    float w[2 * kFilterR + 1][2 * kFilterR + 1][kFilterR + 1] = {};
+    for (auto &row : half)
+        for (int &h : row) h = -1;
+    for (int q = 0; q < st.n; ++q) {
+        const int di = (int8_t)(st.off[q] & 0xff), dj = (int8_t)((st.off[q] >> 8) & 0xff);
+        const int dk = abs((int8_t)((st.off[q] >> 16) & 0xff));
+        int &h = half[di + kFilterR][dj + kFilterR];
+        h = dk > h ? dk : h;
+        w[di + kFilterR][dj + kFilterR][dk] = st.w[q];
+        R = std::max(R, std::max(abs(di), std::max(abs(dj), dk)));
+    }
+    memset(F, 0, sizeof *F);
+    for (int h = 0; h <= kFilterR; ++h) {
+        F->start[h] = n;
+        for (int i = 0; i <= 2 * kFilterR; ++i)
+            for (int j = 0; j <= 2 * kFilterR; ++j) {
+                if (half[i][j] != h) continue;
+                F->di[n] = (short)(i - kFilterR);
+                F->dj[n] = (short)(j - kFilterR);
+                memcpy(F->w[n], w[i][j], sizeof F->w[n]);
+                ++n;
+            }
+    }
+    F->start[kFilterR + 1] = n;
+    return R;
+}
+
+// A block's tile of outputs: ti x tj rows of kt threads, four elements along z each.
+struct FilterTile {
+    int ti, tj, kt, nbj, nbk;
+};
+
+// s + c += the columns of half-extent H and above of the four elements whose window starts at t.
+template <int R, int H>
+__device__ __forceinline__ void filter_cols(const FilterCols &F, const float *t, int SJ, int SK, float (&s)[4],
+                                            float (&c)[4]) {
+#pragma unroll 1
+    for (int q = F.start[H]; q < F.start[H + 1]; ++q) {
+        constexpr int lo = (R - H) & ~3, n4 = (R + H + 4 - lo + 3) / 4;
+        const float4 *row = (const float4 *)(t + (F.di[q] * SJ + F.dj[q]) * SK + lo);
+        float v[4 * n4];
+#pragma unroll
+        for (int i = 0; i < n4; ++i) {
+            const float4 x = row[i];
+            v[4 * i] = x.x;
+            v[4 * i + 1] = x.y;
+            v[4 * i + 2] = x.z;
+            v[4 * i + 3] = x.w;
+        }
+#pragma unroll
+        for (int d = -H; d <= H; ++d) {
+            const float w = F.w[q][d < 0 ? -d : d];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                float e;
+                two_sum(s[m], __fmul_rn(w, v[m + R + d - lo]), s[m], e);
+                c[m] += e;
+            }
+        }
+    }
+    if constexpr (H < R) filter_cols<R, H + 1>(F, t, SJ, SK, s, c);
+}
+
 // mode 0: out = (sum w v) / hs[e] (hs nullable: computed);  mode 1: out = sum w v/hs[e2];
 // mode 2 (hs): out = sum w over in-bounds neighbours. preserved (mode 0): out = 1 there.
-__global__ void __launch_bounds__(256) filter_kernel(int nx, int ny, int nz, const FastDiv fy, const FastDiv fz,
-                                                     const Stencil st, int mode,
+// FP32 products summed with their rounding errors (a few ulp whatever the stencil, up to ~900 terms at
+// rmin 6). Bound by FP32 issue, eight operations per tap. v, v/hs or one (zero outside the grid) of the
+// tile and its margin R goes to shared memory once, and a thread takes four elements along z, so that a
+// column of taps costs it two or three 16-byte loads. A bounds test, a global load, the division and the
+// sum of weights (wanted or not) at every tap took 209 us at 192x96x96 with rmin 3 where this takes 69.
+// Plain FP32 sums along a column would take a third of the operations, but moved the compliance of a
+// twelve-step SIMP run at 20x8x8 by 7e-6.
+template <int R>
+__global__ void __launch_bounds__(256) filter_kernel(int nx, int ny, int nz, const __grid_constant__ FilterTile T,
+                                                     const __grid_constant__ FilterCols F, int mode,
                                                      const float *__restrict__ hs, const float *__restrict__ in,
-                                                     const uint8_t *__restrict__ preserved, float *out) {
-    const int64_t n_elem = (int64_t)nx * ny * nz;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_elem; e += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        unflatten3((uint32_t)e, fy, fz, i, j, k);
-        // FP32 with compensated (Neumaier) summation in the fixed stencil order: error of a
-        // few ulp whatever the stencil size (up to ~900 terms at rmin 6).
-        float s = 0.0f, sc = 0.0f, ws = 0.0f, wc = 0.0f;
-        // Away from the x and y faces only z can leave the grid: the same terms in the same
-        // order, with one z test and a precomputed flat offset per term (a warp's elements
-        // lie in one or two z columns, so the branch rarely splits a warp).
-        if (st.flat && i >= st.r && i < nx - st.r && j >= st.r && j < ny - st.r) {
-            for (int q = 0; q < st.n; ++q) {
-                const int k2 = k + (int)(int8_t)((st.off[q] >> 16) & 0xff);
-                if (k2 < 0 || k2 >= nz) continue;
-                const int64_t e2 = e + st.doff[q];
-                const float w = st.w[q];
-                neumaier_add(ws, wc, w);
-                if (mode == 0) neumaier_add(s, sc, w * in[e2]);
-                else if (mode == 1) neumaier_add(s, sc, w * (in[e2] / hs[e2]));
-            }
-        } else {
-            for (int q = 0; q < st.n; ++q) {
-                int di, dj, dk;
-                unpack_off(st.off[q], di, dj, dk);
-                const int i2 = i + di, j2 = j + dj, k2 = k + dk;
-                if (i2 < 0 || i2 >= nx || j2 < 0 || j2 >= ny || k2 < 0 || k2 >= nz) continue;
-                const int64_t e2 = ((int64_t)i2 * ny + j2) * nz + k2;
-                const float w = st.w[q];
-                neumaier_add(ws, wc, w);
-                if (mode == 0) neumaier_add(s, sc, w * in[e2]);
-                else if (mode == 1) neumaier_add(s, sc, w * (in[e2] / hs[e2]));
+                                                     const uint8_t *__restrict__ preserved, float *__restrict__ out) {
+    extern __shared__ float4 tile4[];
+    float *tile = (float *)tile4;
+    const int SK = (4 * T.kt + 2 * R + 3) & ~3, SJ = T.tj + 2 * R, rows = (T.ti + 2 * R) * SJ;
+    const int bk = blockIdx.x % T.nbk, bij = blockIdx.x / T.nbk, bj = bij % T.nbj, bi = bij / T.nbj;
+    const int i0 = bi * T.ti, j0 = bj * T.tj, k0 = bk * 4 * T.kt;
+    const int tid = threadIdx.x, lane = tid & 31, kt = tid % T.kt, ij = tid / T.kt, jl = ij % T.tj, il = ij / T.tj;
+    float s[4], c[4], h[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+    const bool own = mode == 0 && hs == nullptr;  // the sums of weights first
+    for (int pass = own ? 0 : 1; pass < 2; ++pass) {
+        const bool ones = mode == 2 || pass == 0;
+#pragma unroll 4
+        for (int r = tid >> 5; r < rows; r += (int)blockDim.x >> 5) {
+            const int a = r / SJ, i = i0 + a - R, j = j0 + (r - a * SJ) - R;
+            const bool in_ij = i >= 0 && i < nx && j >= 0 && j < ny;
+            const int64_t e = ((int64_t)i * ny + j) * nz;
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int kk = lane + 32 * p, k = k0 + kk - R;
+                if (kk >= SK) continue;
+                float v = 0.0f;
+                if (in_ij && k >= 0 && k < nz) {
+                    if (ones) v = 1.0f;
+                    else if (mode == 1) v = in[e + k] / hs[e + k];
+                    else v = in[e + k];
+                }
+                tile[r * SK + kk] = v;
             }
         }
-        s += sc;
-        ws += wc;
-        float o;
-        if (mode == 0) {
-            const float h = hs ? hs[e] : ws;
-            o = s / h;
-            if (preserved && preserved[e]) o = 1.0f;
-        } else if (mode == 1) {
-            o = (float)s;
-        } else {
-            o = (float)ws;
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < 4; ++m) s[m] = c[m] = 0.0f;
+        filter_cols<R, 0>(F, tile + ((il + R) * SJ + jl + R) * SK + 4 * kt, SJ, SK, s, c);
+        if (pass == 0) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) h[m] = s[m] + c[m];
+            __syncthreads();
         }
-        out[e] = o;
+    }
+    const int i = i0 + il, j = j0 + jl, k = k0 + 4 * kt;
+    if (i >= nx || j >= ny || k >= nz) return;
+    const int64_t e = ((int64_t)i * ny + j) * nz + k;
+    float o[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        o[m] = s[m] + c[m];
+        if (mode == 0 && k + m < nz) {
+            o[m] = o[m] / (own ? h[m] : hs[e + m]);
+            if (preserved && preserved[e + m]) o[m] = 1.0f;
+        }
+    }
+    if ((nz & 3) == 0 && ((uintptr_t)out & 15) == 0) {
+        *(float4 *)(out + e) = make_float4(o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            if (k + m < nz) out[e + m] = o[m];
     }
 }
 
@@ -290,15 +359,48 @@ static unsigned elem_blocks(const gbsimp_ctx *ctx, int64_t n, int threads) {
     return (unsigned)(b < 1 ? 1 : b);
 }
 
+// The tile: 4 kt elements along z (kt a power of two up to 8 that covers nz), then the split of the
+// rows of 256, 128 or 64 threads with the fewest elements to load; the smaller blocks only where the
+// larger would leave SMs without one.
+static FilterTile filter_tile(const gbsimp_ctx *ctx, int nx, int ny, int nz, int R, int *threads) {
+    auto up = [](int a, int b) { return (a + b - 1) / b; };
+    FilterTile T{1, 1, 1, 1, 1};
+    while (T.kt < 8 && 4 * T.kt < nz) T.kt *= 2;
+    T.nbk = up(nz, 4 * T.kt);
+    const int sms = ctx->num_sms > 0 ? ctx->num_sms : 148;
+    for (int nt = 256; nt >= 64; nt /= 2) {
+        double best = 1e300;
+        for (int ti = 1; ti <= nt / T.kt; ti *= 2) {
+            const int tj = nt / T.kt / ti;
+            const double rows = (double)(ti + 2 * R) * (tj + 2 * R);
+            const double load = rows * up(nx, ti) * up(ny, tj);
+            if (rows * ((4 * T.kt + 2 * R + 3) & ~3) * 4 > 48 * 1024 || load >= best) continue;
+            best = load;
+            T.ti = ti;
+            T.tj = tj;
+        }
+        *threads = nt;
+        T.nbj = up(ny, T.tj);
+        if ((int64_t)up(nx, T.ti) * T.nbj * T.nbk >= sms) break;
+    }
+    return T;
+}
+
 int filter_launch(const gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin, int mode, const float *hs,
                   const float *in, const uint8_t *preserved, float *out, cudaStream_t st) {
     Stencil s;
     int rc = make_stencil(rmin, &s);
     if (rc) return rc;
-    set_flat_offsets(ny, nz, &s);
-    const int64_t n = (int64_t)nx * ny * nz;
-    filter_kernel<<<elem_blocks(ctx, n, 256), 256, 0, st>>>(nx, ny, nz, fast_div(ny), fast_div(nz), s, mode, hs, in,
-                                                            preserved, out);
+    FilterCols F;
+    const int R = filter_columns(s, &F);
+    int nt = 256;
+    const FilterTile T = filter_tile(ctx, nx, ny, nz, R, &nt);
+    const unsigned blocks = (unsigned)(((nx + T.ti - 1) / T.ti) * T.nbj * T.nbk);
+    const size_t smem = sizeof(float) * (size_t)(T.ti + 2 * R) * (T.tj + 2 * R) * ((4 * T.kt + 2 * R + 3) & ~3);
+    static void (*const kern[])(int, int, int, FilterTile, FilterCols, int, const float *, const float *,
+                                const uint8_t *, float *) = {filter_kernel<0>, filter_kernel<1>, filter_kernel<2>,
+                                                             filter_kernel<3>, filter_kernel<4>, filter_kernel<5>};
+    kern[R]<<<blocks, nt, smem, st>>>(nx, ny, nz, T, F, mode, hs, in, preserved, out);
     GBS_LAUNCH_CHECK("filter_kernel");
     return GBS_OK;
 }
