@@ -221,6 +221,21 @@ __device__ __forceinline__ void block_sum_df(df32 (&v)[K], float2 *scratch) {
     }
 }
 
+// Packets: 16-byte accesses at the GPU's coherence point, three values and an epoch that a reader polls.
+__device__ __forceinline__ void st_packet(void *p, unsigned a, unsigned b, unsigned c, unsigned ep) {
+    const unsigned long long lo = ((unsigned long long)b << 32) | a, hi = ((unsigned long long)ep << 32) | c;
+    asm volatile("{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }" ::"l"(p), "l"(lo), "l"(hi)
+                 : "memory");
+}
+__device__ __forceinline__ uint4 ld_packet(const void *p) {
+    unsigned long long lo, hi;
+    asm volatile("{ .reg .b128 v; ld.relaxed.gpu.global.b128 v, [%2]; mov.b128 {%0, %1}, v; }"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p)
+                 : "memory");
+    return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
+}
+
 // Division of a grid index n < 2^31 by a fixed divisor 1 <= d < 2^31 as a multiply-high, an add
 // and a shift (Granlund and Montgomery 1994, round-up method): with l = ceil(log2 d) and
 // m = floor(2^32 (2^l - d) / d) + 1, n / d = (umulhi(n, m) + n) >> l for every n < 2^32 when

@@ -410,9 +410,7 @@ struct OcScalars {
     double l1, l2, lfinal, npres;
     int steps, done;
     unsigned counter;
-    unsigned bar;  // grid barrier of oc_coop_kernel (monotonic within one call)
-    int status;    // GBS_ETIMEOUT when a barrier wait of oc_coop_kernel ran out
-    int pad;
+    int status;  // GBS_ETIMEOUT when a wait of oc_coop_kernel ran out
 };
 
 struct OcParams {
@@ -485,11 +483,13 @@ __device__ __forceinline__ float oc_trial(float x, float dc, float inv_l, const 
 }
 
 __global__ void oc_init_kernel(int64_t n, const OcParams P, const float *__restrict__ dc, double *partials,
-                               OcScalars *sc) {
+                               OcScalars *sc, uint4 *box, int packets) {
     sc->done = 0;  // every block writes the same values
     sc->steps = 0;
-    sc->bar = 0;
     sc->status = 0;
+    // oc_coop_kernel's packets: none may carry an epoch of the rounds to come
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < packets; i += gridDim.x * blockDim.x)
+        box[i] = make_uint4(0, 0, 0, 0);
     if (P.l2 >= 0.0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             sc->l1 = P.l1;
@@ -662,46 +662,79 @@ __global__ void __launch_bounds__(kOcThreads) oc_multi_kernel(int64_t n, const O
     }
 }
 
-__device__ __forceinline__ unsigned long long oc_now_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
+// ---- multisection in one cooperative launch ----------------------------------------------
+// The rounds of oc_multi_kernel without a launch per round, one block per SM. Per element a trial density
+// is a clamp of a line in sqrt(1 / mid), a + d sat(p sqrt(1 / mid) + q): its five numbers are formed
+// once and kept in shared memory (the rest, beyond 2 M elements on 152 SMs, anew in every round), so that
+// a trial takes two operations. A block's sums of the kOcNodes trial volumes and of w a go to the first
+// block as packets; it adds them in block order, walks the tree and sends (l1, l2, lfinal, steps, done)
+// back. Its polls are the only ones on the sums; one block (up to kOcShare elements) has no exchange.
+// Bound by the latency of its rounds: 61x37x23 takes 38 us and 192x96x96 (1.8 M elements) 68, where a grid
+// barrier, all blocks adding all sums, and trials of six operations from global memory took 50 and
+// 125. A wait that runs out sets sc->status = GBS_ETIMEOUT and ends the rounds; the host reports it.
+constexpr int kCoopThreads = 512;
+constexpr int kCoopRow = kCoopThreads + 16;  // a node's row of partial sums: two rows meet in no bank
+constexpr int kCoopPer = 13;                 // packets a lane of the first block waits for
+constexpr int kCoopBlocks = 16 * kCoopPer;
+constexpr int kCoopCopies = 8;               // of the first block's answer
+constexpr int kOcShare = 4 * kCoopThreads;   // elements per block below one block per SM
+constexpr size_t kCoopBoxAt = 16384;         // bytes into the partials, behind oc_init_kernel's
+constexpr size_t kCoopSums = sizeof(float) * (kOcNodes + 1) * kCoopRow;
+constexpr int kCoopKeep = (int)((220 * 1024 - kCoopSums) / (3 * sizeof(float) * kCoopThreads));
+static_assert(kOcNodes + 1 == 32 && kCoopThreads == 16 * 32, "sixteen lanes per node");
+static_assert(kCoopBoxAt + 16 * ((size_t)32 * kCoopBlocks + 3 * kCoopCopies) <= 4 * 4096 * sizeof(double), "room");
+static int coop_packets(int nblk) { return nblk > 1 ? 32 * nblk + 3 * kCoopCopies : 0; }
+
+// p, q and w d of an element; base gains w a.
+__device__ __forceinline__ float3 oc_line(float xe, float dce, float we, bool pre, const OcParams &P, float sfloor,
+                                          float &base) {
+    if (pre) {  // xnew = 1
+        base += we;
+        return make_float3(0.0f, 0.0f, 0.0f);
+    }
+    const float lo = xe - P.move, hi = xe + P.move, b = fminf(fmaxf(1.0f, lo), hi);
+    const float a = fminf(fmaxf(xe * sfloor, fminf(fmaxf(0.0f, lo), hi)), b), d = b - a;
+    base = fmaf(we, a, base);
+    const float inv = d > 0.0f ? 1.0f / d : 0.0f;
+    return make_float3(xe * sqrtf(fmaxf(-dce, 0.0f)) * inv, -a * inv, we * d);
 }
 
-// ---- multisection in one cooperative launch ----------------------------------------------
-// The rounds of oc_multi_kernel without a launch per round. In each round every block
-// evaluates the kOcNodes trial volumes on its elements and publishes its block sums (slot
-// round & 1: a block rewrites a slot only after every block has left the barrier that read it),
-// arrives on a monotonic counter and waits, bounded in time, for all blocks; then every block
-// sums all partials in block order and walks the tree itself, so that all blocks hold the same
-// (l1, l2, lfinal, steps, done) and no broadcast is needed. After the last round each block
-// writes xnew for its elements (oc_final_kernel's step). A wait that runs out sets
-// sc->status = GBS_ETIMEOUT and ends the rounds; the host reports it.
-__global__ void __launch_bounds__(kOcThreads) oc_coop_kernel(int64_t n, const OcParams P, const float *__restrict__ x,
-                                                             const float *__restrict__ dc,
-                                                             const uint8_t *__restrict__ pres,
-                                                             const float *__restrict__ w, float2 *partials,
-                                                             OcScalars *sc, float *xnew, unsigned long long wait_ns) {
+__global__ void __launch_bounds__(kCoopThreads, 1)
+    oc_coop_kernel(int64_t n, const OcParams P, const float *__restrict__ x, const float *__restrict__ dc,
+                   const uint8_t *__restrict__ pres, const float *__restrict__ w, uint4 *box, OcScalars *sc,
+                   float *xnew, int keep, unsigned polls) {
+    extern __shared__ float coop_sh[];
+    float *s_part = coop_sh, *kp = s_part + (kOcNodes + 1) * kCoopRow, *kq = kp + keep, *kw = kq + keep;
     __shared__ float s_sq[kOcNodes];
-    __shared__ bool s_stop[kOcNodes];
+    __shared__ int s_stop[kOcNodes];
     __shared__ double s_mid[kOcNodes];
-    __shared__ float s_part[kOcNodes][kOcThreads + 8];  // rows padded: conflict-free column sums
-    __shared__ double s_tot[kOcNodes];
-    __shared__ double s_l1, s_l2, s_lfinal;
+    __shared__ double s_tot[kOcNodes + 1];
+    __shared__ double s_lim[3];  // l1, l2, lfinal
     __shared__ int s_steps, s_done, s_ok;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nblk = gridDim.x, bid = blockIdx.x;
+    uint4 *answer = box + 32 * nblk;
     if (tid == 0) {
-        s_l1 = sc->l1;
-        s_l2 = sc->l2;
-        s_lfinal = sc->lfinal;
+        s_lim[0] = sc->l1;
+        s_lim[1] = sc->l2;
+        s_lim[2] = sc->lfinal;
         s_steps = sc->steps;
         s_done = sc->done;
         s_ok = 1;
     }
-    __syncthreads();
     const float sfloor = sqrtf(P.sqrt_floor);
     const double target = P.volfrac * (double)n - sc->npres;  // vol > volfrac <=> sum > target
+    const int64_t first = (int64_t)bid * kCoopThreads + tid, stride = (int64_t)nblk * kCoopThreads;
+    // the kept elements of this thread: only it reads them back
+    float kept = 0.0f;
+    int nk = 0;
+    for (int64_t e = first; e < n && nk * kCoopThreads < keep; e += stride, ++nk) {
+        const float3 l = oc_line(x[e], dc[e], w[e], pres && pres[e], P, sfloor, kept);
+        kp[nk * kCoopThreads + tid] = l.x;
+        kq[nk * kCoopThreads + tid] = l.y;
+        kw[nk * kCoopThreads + tid] = l.z;
+    }
+    __syncthreads();
     // Rounds have two shapes. While l1 is still 0 the bisection's midpoints are l2/2, l2/4, ...
     // for as long as every volume stays at or below the target (each step sets l2 = mid); a
     // chain round evaluates the next kOcNodes midpoints of that all-left path, formed exactly
@@ -709,16 +742,19 @@ __global__ void __launch_bounds__(kOcThreads) oc_coop_kernel(int64_t n, const Oc
     // l1 > 0, tree rounds evaluate the full kOcLevels-level tree. Each round advances the
     // bisection by at least one step, so max_bisect rounds bound the loop.
     for (int round = 0; round < P.max_bisect; ++round) {
-        if (s_done || !s_ok) break;  // block-uniform: written before the last __syncthreads
-        const bool chain = s_l1 == 0.0;
-        if (tid < kOcNodes) {
-            double lo = s_l1, hi = s_l2;
+        // block-uniform: written before the last __syncthreads. Through a shuffle, so that the compiler
+        // knows it uniform: in code it takes for divergent every shuffle costs about 250 cycles
+        if (__shfl_sync(0xffffffffu, (int)(s_done != 0 || s_ok == 0), 0)) break;
+        const bool chain = s_lim[0] == 0.0;
+        const unsigned ep = (unsigned)round + 1;
+        if (warp < 2 && lane < kOcNodes) {
+            double lo = s_lim[0], hi = s_lim[1];
             if (chain) {
-                // tid halvings 0.5 (hi + 0) of the all-left path: exact, so the same bits as that
+                // halvings 0.5 (hi + 0) of the all-left path: exact, so the same bits as that
                 // loop of dependent FP64 operations (l2 <= 1e9 stays far above the subnormals)
-                hi = ldexp(hi, -tid);
+                hi = ldexp(hi, -lane);
             } else {
-                const int path = tid + 1, depth = 31 - __clz(path);
+                const int path = lane + 1, depth = 31 - __clz(path);
                 for (int i = depth - 1; i >= 0; --i) {
                     const double m = 0.5 * (hi + lo);
                     if ((path >> i) & 1)
@@ -727,140 +763,155 @@ __global__ void __launch_bounds__(kOcThreads) oc_coop_kernel(int64_t n, const Oc
                         hi = m;
                 }
             }
-            const double m = 0.5 * (hi + lo);
-            s_mid[tid] = m;
-            s_sq[tid] = (float)sqrt(1.0 / m);
-            s_stop[tid] = (hi - lo) / (lo + hi + P.tol_eps) < P.tol;
+            if (warp == 0) {
+                const double m = 0.5 * (hi + lo);
+                s_mid[lane] = m;
+                s_sq[lane] = (float)sqrt(1.0 / m);
+            } else {
+                s_stop[lane] = (hi - lo) / (lo + hi + P.tol_eps) < P.tol;
+            }
         }
         __syncthreads();
-        float sq[kOcNodes], v[kOcNodes];
+        float sq[kOcNodes], v[kOcNodes], base = kept;
 #pragma unroll
         for (int t = 0; t < kOcNodes; ++t) {
             sq[t] = s_sq[t];
             v[t] = 0.0f;
         }
-        for (int64_t e = bid * (int64_t)kOcThreads + tid; e < n; e += (int64_t)nblk * kOcThreads) {
-            const float we = w[e];
-            if (pres && pres[e]) {
+        auto trials = [&](float p, float q, float wd) {
 #pragma unroll
-                for (int t = 0; t < kOcNodes; ++t) v[t] += we;
-                continue;
-            }
-            const float xe = x[e], s0 = sqrtf(fmaxf(-dc[e], 0.0f));
-            const float lo = xe - P.move, hi = xe + P.move;
-#pragma unroll
-            for (int t = 0; t < kOcNodes; ++t) {
-                float tv = xe * fmaxf(s0 * sq[t], sfloor);
-                tv = fminf(fmaxf(tv, 0.0f), 1.0f);
-                tv = fminf(fmaxf(tv, lo), hi);
-                v[t] = fmaf(we, tv, v[t]);
-            }
+            for (int t = 0; t < kOcNodes; ++t) v[t] = fmaf(wd, __saturatef(fmaf(p, sq[t], q)), v[t]);
+        };
+#pragma unroll 2
+        for (int k = 0; k < nk; ++k)
+            trials(kp[k * kCoopThreads + tid], kq[k * kCoopThreads + tid], kw[k * kCoopThreads + tid]);
+        for (int64_t e = first + (int64_t)nk * stride; e < n; e += stride) {
+            const float3 l = oc_line(x[e], dc[e], w[e], pres && pres[e], P, sfloor, base);
+            trials(l.x, l.y, l.z);
         }
 #pragma unroll
-        for (int t = 0; t < kOcNodes; ++t) s_part[t][tid] = v[t];
+        for (int t = 0; t < kOcNodes; ++t) s_part[t * kCoopRow + tid] = v[t];
+        s_part[kOcNodes * kCoopRow + tid] = base;
         __syncthreads();
-        // block sums: node t = tid / 8 summed by the 8 lanes tid % 8 (columns sub, sub + 8, ...),
-        // then across those lanes; every sum in a fixed order
-        float2 *part = partials + (size_t)(round & 1) * kOcNodes * nblk;
-        const int t8 = tid >> 3, sub = tid & 7;
-        {
-            df32 a{0.0f, 0.0f};
-            if (t8 < kOcNodes)
+        // block sums: node t summed by 16 lanes (columns sub, sub + 16, ...), then across those lanes; the
+        // sums' errors carried; every sum in a fixed order
+        const int t = tid >> 4, sub = tid & 15;
+        ddv a{0.0f, 0.0f};
 #pragma unroll 8
-                for (int j = sub; j < kOcThreads; j += 8) a = df_add(a, df32{s_part[t8][j], 0.0f});
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1)
-                a = df_add(a, df32{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)});
-            if (t8 < kOcNodes && sub == 0) part[t8 * nblk + bid] = make_float2(a.hi, a.lo);
+        for (int j = sub; j < kCoopThreads; j += 16) {
+            float e;
+            two_sum(a.h, s_part[t * kCoopRow + j], a.h, e);
+            a.l += e;
         }
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            atomicAdd(&sc->bar, 1u);
-            const unsigned goal = (unsigned)nblk * (unsigned)(round + 1);
-            const unsigned long long t0 = oc_now_ns();
-            while (*(volatile unsigned *)&sc->bar < goal) {
-                if (oc_now_ns() - t0 > wait_ns) {
-                    s_ok = 0;
-                    atomicExch(&sc->status, (int)GBS_ETIMEOUT);
-                    break;
+        auto across = [&]() {
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+                a = dd_add(a, ddv{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)});
+        };
+        across();
+        bool ok = true;
+        if (nblk > 1) {
+            if (sub == 0) st_packet(box + t * nblk + bid, __float_as_uint(a.h), __float_as_uint(a.l), 0, ep);
+            if (bid == 0) {
+                float2 pv[kCoopPer];
+                unsigned need = 0;
+#pragma unroll
+                for (int m = 0; m < kCoopPer; ++m) {
+                    pv[m] = make_float2(0.0f, 0.0f);
+                    if (sub + 16 * m < nblk) need |= 1u << m;
                 }
-                __nanosleep(64);
+                for (unsigned sweep = 0; need != 0; ++sweep) {
+                    if (sweep >= polls) {
+                        ok = false;
+                        break;
+                    }
+#pragma unroll
+                    for (int m = 0; m < kCoopPer; ++m)
+                        if ((need >> m) & 1u) {
+                            const uint4 u = ld_packet(box + t * nblk + sub + 16 * m);
+                            if (u.w == ep) {
+                                pv[m] = make_float2(__uint_as_float(u.x), __uint_as_float(u.y));
+                                need &= ~(1u << m);
+                            }
+                        }
+                }
+                __syncwarp();
+                a = ddv{pv[0].x, pv[0].y};
+#pragma unroll
+                for (int m = 1; m < kCoopPer; ++m) a = dd_add(a, ddv{pv[m].x, pv[m].y});
+                across();
+            } else if (tid < 3) {
+                uint4 u = ld_packet(answer + 3 * (bid & (kCoopCopies - 1)) + tid);
+                for (unsigned sweep = 0; u.w != ep; ++sweep) {
+                    if (sweep >= polls) {
+                        ok = false;
+                        break;
+                    }
+                    u = ld_packet(answer + 3 * (bid & (kCoopCopies - 1)) + tid);
+                }
+                s_lim[tid] = __hiloint2double((int)u.y, (int)u.x);
+                if (tid == 0) {
+                    s_steps = (int)(u.z >> 1);
+                    s_done = (int)(u.z & 1u);
+                }
             }
-            __threadfence();
+            if (!ok) s_ok = 0;
         }
-        __syncthreads();
-        if (!s_ok) break;
-        // totals, the same way over the blocks' partials (loads issued eight at a time, added in
-        // block order)
-        {
-            df32 a{0.0f, 0.0f};
-            if (t8 < kOcNodes) {
-                const float2 *pt = part + t8 * nblk;
-                int b = sub;
-                for (; b + 56 < nblk; b += 64) {
-                    float2 pv[8];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) pv[q] = __ldcg(&pt[b + 8 * q]);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) a = df_add(a, df32{pv[q].x, pv[q].y});
+        if (bid == 0) {
+            if (sub == 0) s_tot[t] = dd_value(a);
+            __syncthreads();
+            if (warp == 0) {  // bisection's tests along the chain or the tree (oc_multi_kernel's walk)
+                const bool node = lane < kOcNodes;
+                const unsigned right = __ballot_sync(0xffffffffu, node && s_tot[node ? lane : 0] + s_tot[kOcNodes] > target);
+                const unsigned stop = __ballot_sync(0xffffffffu, node && s_stop[node ? lane : 0]);
+                int steps = s_steps, done = 0, at = 0, n1 = -1, n2 = -1, nf = 0;
+                for (int lvl = 0; lvl < (chain ? kOcNodes : kOcLevels); ++lvl) {
+                    nf = at;
+                    ++steps;
+                    if ((stop >> at) & 1u) {
+                        done = 1;
+                        break;
+                    }
+                    const bool r = (right >> at) & 1u;
+                    if (r)
+                        n1 = at;
+                    else
+                        n2 = at;
+                    at = r ? 2 * at + 2 : (chain ? at + 1 : 2 * at + 1);
+                    if (steps >= P.max_bisect) {
+                        done = 1;
+                        break;
+                    }
+                    if (chain && r) break;  // off the all-left path: tree rounds from here
                 }
-                for (; b < nblk; b += 8) {
-                    const float2 p = __ldcg(&pt[b]);
-                    a = df_add(a, df32{p.x, p.y});
+                if (lane < 3) {
+                    const int from = lane == 0 ? n1 : (lane == 1 ? n2 : nf);
+                    if (from >= 0) s_lim[lane] = s_mid[from];
+                }
+                if (lane == 0) {
+                    s_steps = steps;
+                    s_done = done;
+                }
+                __syncwarp();
+                if (nblk > 1 && s_ok && lane < 3 * kCoopCopies) {
+                    const double l = s_lim[lane % 3];
+                    st_packet(answer + lane, (unsigned)__double2loint(l), (unsigned)__double2hiint(l),
+                              (unsigned)steps << 1 | (unsigned)done, ep);
                 }
             }
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1)
-                a = df_add(a, df32{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)});
-            if (t8 < kOcNodes && sub == 0) s_tot[t8] = df_value(a);
-        }
-        __syncthreads();
-        if (tid == 0) {  // bisection's tests along the chain or the tree (oc_multi_kernel's walk)
-            double l1 = s_l1, l2 = s_l2, lfinal = s_lfinal;
-            int steps = s_steps, done = 0, node = 0;
-            for (int lvl = 0; lvl < (chain ? kOcNodes : kOcLevels); ++lvl) {
-                const double m = s_mid[node];
-                if (s_stop[node]) {
-                    lfinal = m;
-                    steps += 1;
-                    done = 1;
-                    break;
-                }
-                const bool right = s_tot[node] > target;
-                if (right) {
-                    l1 = m;
-                    node = 2 * node + 2;
-                } else {
-                    l2 = m;
-                    node = chain ? node + 1 : 2 * node + 1;
-                }
-                lfinal = m;
-                steps += 1;
-                if (steps >= P.max_bisect) {
-                    done = 1;
-                    break;
-                }
-                if (chain && right) break;  // off the all-left path: tree rounds from here
-            }
-            s_l1 = l1;
-            s_l2 = l2;
-            s_lfinal = lfinal;
-            s_steps = steps;
-            s_done = done;
         }
         __syncthreads();
     }
+    if (tid == 0 && !s_ok) atomicExch(&sc->status, (int)GBS_ETIMEOUT);
     if (bid == 0 && tid == 0) {
-        sc->l1 = s_l1;
-        sc->l2 = s_l2;
-        sc->lfinal = s_lfinal;
+        sc->l1 = s_lim[0];
+        sc->l2 = s_lim[1];
+        sc->lfinal = s_lim[2];
         sc->steps = s_steps;
         sc->done = s_done;
     }
-    const float inv_l = (float)(1.0 / s_lfinal);
-    for (int64_t e = bid * (int64_t)kOcThreads + tid; e < n; e += (int64_t)nblk * kOcThreads)
-        xnew[e] = oc_trial(x[e], dc[e], inv_l, P, pres && pres[e]);
+    const float inv_l = (float)(1.0 / s_lim[2]);
+    for (int64_t e = first; e < n; e += stride) xnew[e] = oc_trial(x[e], dc[e], inv_l, P, pres && pres[e]);
 }
 
 __global__ void oc_final_kernel(int64_t n, const OcParams P, const float *__restrict__ x,
@@ -967,24 +1018,22 @@ int oc_prepare_impl(const gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin, 
 }
 
 // Blocks of oc_coop_kernel that can be resident together on the context's device (cached per
-// device), capped by the partials room; 0 when cooperative launches are unavailable.
+// device): one per SM; 0 when cooperative launches are unavailable.
 static int oc_coop_blocks(const gbsimp_ctx *ctx) {
     static std::atomic<int> cache[64];
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64) return 0;
     int v = cache[dev].load(std::memory_order_relaxed);
     if (v != 0) return v > 0 ? v : 0;
-    int coop = 0, per_sm = 0;
+    int coop = 0;
+    const int most = (int)(kCoopSums + 3 * sizeof(float) * kCoopThreads * kCoopKeep);
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, oc_coop_kernel, kOcThreads, 0) != cudaSuccess ||
-        per_sm < 1) {
+        cudaFuncSetAttribute(oc_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) {
         (void)cudaGetLastError();
         cache[dev].store(-1, std::memory_order_relaxed);
         return 0;
     }
-    constexpr int kRoom = (4 * 4096 * (int)sizeof(double)) / (2 * kOcNodes * (int)sizeof(float2));
-    v = per_sm * (ctx->num_sms > 0 ? ctx->num_sms : 148);
-    v = v < kRoom ? v : kRoom;
+    v = std::min(ctx->num_sms > 0 ? ctx->num_sms : 148, kCoopBlocks);
     cache[dev].store(v, std::memory_order_relaxed);
     return v;
 }
@@ -1004,20 +1053,21 @@ int oc_run_impl(const gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin, cons
     P.l2 = prm->l2;
     P.max_bisect = prm->max_bisect;
     const unsigned blocks = reduce_blocks(ctx, n, 256);
-    oc_init_kernel<<<blocks, 256, 0, st>>>(n, P, dc, w.partials, w.sc);
-    GBS_LAUNCH_CHECK("oc_init_kernel");
-    // One cooperative launch for the multisection and xnew when its blocks can be resident
-    // together (two slots of kOcNodes double-float partials per block fit the workspace).
+    // One cooperative launch for the multisection and xnew. A block takes kOcShare elements before there is
+    // one on every SM: fewer blocks make the exchange cheaper than the trials get dearer.
     const int cb = oc_coop_blocks(ctx);
+    const int nb = (int)std::min<int64_t>((n + kOcShare - 1) / kOcShare, cb);
+    uint4 *box = (uint4 *)((char *)w.partials + kCoopBoxAt);
+    oc_init_kernel<<<blocks, 256, 0, st>>>(n, P, dc, w.partials, w.sc, box, coop_packets(nb));
+    GBS_LAUNCH_CHECK("oc_init_kernel");
     if (cb > 0) {
-        int64_t nb = (n + kOcThreads - 1) / kOcThreads;
-        nb = nb > cb ? cb : (nb < 1 ? 1 : nb);
-        float2 *parts = (float2 *)w.partials;
-        unsigned long long wait_ns = 2000000000ull;  // 2 s per barrier wait
+        const int64_t per = (n + (int64_t)nb * kCoopThreads - 1) / ((int64_t)nb * kCoopThreads);
+        int keep = (int)std::min<int64_t>(per, kCoopKeep) * kCoopThreads;
+        unsigned polls = 1u << 22;  // per wait; a poll is an L2 round trip, so two seconds or so
         void *args[] = {(void *)&n, (void *)&P, (void *)&x, (void *)&dc, (void *)&preserved, (void *)&w.w,
-                        (void *)&parts, (void *)&w.sc, (void *)&xnew, (void *)&wait_ns};
-        GBS_CUDA_TRY(cudaLaunchCooperativeKernel((void *)oc_coop_kernel, dim3((unsigned)nb), dim3(kOcThreads), args, 0,
-                                                 st));
+                        (void *)&box, (void *)&w.sc, (void *)&xnew, (void *)&keep, (void *)&polls};
+        GBS_CUDA_TRY(cudaLaunchCooperativeKernel((void *)oc_coop_kernel, dim3((unsigned)nb), dim3(kCoopThreads), args,
+                                                 kCoopSums + 3 * sizeof(float) * keep, st));
         GBS_LAUNCH_CHECK("oc_coop_kernel");
         return filter_launch(ctx, nx, ny, nz, rmin, 0, w.hs, xnew, preserved, xphys, st);
     }

@@ -64,20 +64,6 @@ struct ChipTable {
 };
 static_assert(sizeof(ChipTable) + 128 <= 4096, "kernel parameters");
 
-// 16-byte accesses at the GPU's coherence point.
-__device__ __forceinline__ void st_packet(void *p, unsigned a, unsigned b, unsigned c, unsigned ep) {
-    const unsigned long long lo = ((unsigned long long)b << 32) | a, hi = ((unsigned long long)ep << 32) | c;
-    asm volatile("{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }" ::"l"(p), "l"(lo), "l"(hi)
-                 : "memory");
-}
-__device__ __forceinline__ uint4 ld_packet(const void *p) {
-    unsigned long long lo, hi;
-    asm volatile("{ .reg .b128 v; ld.relaxed.gpu.global.b128 v, [%2]; mov.b128 {%0, %1}, v; }"
-                 : "=l"(lo), "=l"(hi)
-                 : "l"(p)
-                 : "memory");
-    return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
-}
 // Sums of (h, l) pairs whose leading parts are exact (two-sum) and whose low parts are carried in
 // FP32: a level of a tree waits for one FP32 add, not for a renormalisation.
 // (A rolled loop: the iteration's code has to stay in the instruction cache.)
