@@ -419,7 +419,8 @@ struct OcParams {
     int max_bisect;
 };
 
-// Workspace: [OcScalars (256 B)] [hs: n floats] [w: n floats] [partials: 4*cap doubles]
+// Workspace: [OcScalars (256 B)] [hs: n floats] [w: n floats] [partials: kOcPartials bytes]
+constexpr size_t kOcPartials = 4 * 4096 * sizeof(double) + 65536;
 struct OcWs {
     OcScalars *sc;
     float *hs, *w;
@@ -429,7 +430,7 @@ struct OcWs {
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 static size_t oc_ws_bytes(int64_t n) {
-    return 256 + 2 * align256((size_t)n * sizeof(float)) + align256(4 * 4096 * sizeof(double));
+    return 256 + 2 * align256((size_t)n * sizeof(float)) + align256(kOcPartials);
 }
 
 static OcWs oc_ws(void *ws, int64_t n) {
@@ -663,27 +664,49 @@ __global__ void __launch_bounds__(kOcThreads) oc_multi_kernel(int64_t n, const O
 }
 
 // ---- multisection in one cooperative launch ----------------------------------------------
-// The rounds of oc_multi_kernel without a launch per round, one block per SM. Per element a trial density
-// is a clamp of a line in sqrt(1 / mid), a + d sat(p sqrt(1 / mid) + q): its five numbers are formed
-// once and kept in shared memory (the rest, beyond 2 M elements on 152 SMs, anew in every round), so that
-// a trial takes two operations. A block's sums of the kOcNodes trial volumes and of w a go to the first
-// block as packets; it adds them in block order, walks the tree and sends (l1, l2, lfinal, steps, done)
-// back. Its polls are the only ones on the sums; one block (up to kOcShare elements) has no exchange.
-// Bound by the latency of its rounds: 61x37x23 takes 38 us and 192x96x96 (1.8 M elements) 68, where a grid
-// barrier, all blocks adding all sums, and trials of six operations from global memory took 50 and
-// 125. A wait that runs out sets sc->status = GBS_ETIMEOUT and ends the rounds; the host reports it.
+// The rounds of oc_multi_kernel without a launch per round, one block per SM, six levels (63 midpoints) a
+// round: with tol 1e-4 twelve steps follow the first one to the right, so that three rounds do (with five
+// levels and 31 midpoints along the first path it took five). Per element a trial density is a clamp of a
+// line in sqrt(1 / mid), a + d sat(p sqrt(1 / mid) + q): its numbers are formed once and kept in shared
+// memory (the rest, beyond 2 M elements on 152 SMs, anew in every round), so that a trial takes two
+// operations; half of a block's threads take 32 of the midpoints, half the others. A block's sums of
+// the trial volumes and of w a go to the first block as packets; it adds them in block order, walks the
+// tree and sends (l1, l2, lfinal, steps, done) back. Its polls are the only ones on the sums; one block (up
+// to kOcShare elements) has no exchange. Bound by the latency of its rounds: 61x37x23 takes 24 us and
+// 192x96x96 (1.8 M elements) 61, where a grid barrier, all blocks adding all sums, and trials of six
+// operations from global memory took 50 and 125. A wait that runs out sets sc->status = GBS_ETIMEOUT
+// and ends the rounds; the host reports it.
+constexpr int kCoopLevels = 6;
+constexpr int kCoopNodes = (1 << kCoopLevels) - 1;
 constexpr int kCoopThreads = 512;
-constexpr int kCoopRow = kCoopThreads + 16;  // a node's row of partial sums: two rows meet in no bank
-constexpr int kCoopPer = 13;                 // packets a lane of the first block waits for
-constexpr int kCoopBlocks = 16 * kCoopPer;
-constexpr int kCoopCopies = 8;               // of the first block's answer
-constexpr int kOcShare = 4 * kCoopThreads;   // elements per block below one block per SM
-constexpr size_t kCoopBoxAt = 16384;         // bytes into the partials, behind oc_init_kernel's
-constexpr size_t kCoopSums = sizeof(float) * (kOcNodes + 1) * kCoopRow;
+constexpr int kCoopRow = kCoopThreads / 2 + 8;  // a node's row of partial sums: four rows meet in no bank
+constexpr int kCoopPoll = 10;                   // packets a lane of the first block polls at once
+constexpr int kCoopBlocks = 160;
+constexpr int kCoopCopies = 8;                // of the first block's answer
+constexpr int kOcShare = 4 * kCoopThreads;    // elements per block below one block per SM
+constexpr size_t kCoopBoxAt = 16384;          // bytes into the partials, behind oc_init_kernel's
+constexpr size_t kCoopSums = sizeof(float) * ((kCoopNodes + 1) * kCoopRow + kCoopThreads / 2);
 constexpr int kCoopKeep = (int)((220 * 1024 - kCoopSums) / (3 * sizeof(float) * kCoopThreads));
-static_assert(kOcNodes + 1 == 32 && kCoopThreads == 16 * 32, "sixteen lanes per node");
-static_assert(kCoopBoxAt + 16 * ((size_t)32 * kCoopBlocks + 3 * kCoopCopies) <= 4 * 4096 * sizeof(double), "room");
-static int coop_packets(int nblk) { return nblk > 1 ? 32 * nblk + 3 * kCoopCopies : 0; }
+static_assert(kCoopNodes + 1 == 64 && kCoopThreads == 8 * 64, "eight lanes per node");
+static_assert(kCoopBoxAt + 16 * ((size_t)64 * kCoopBlocks + 3 * kCoopCopies) <= kOcPartials, "room");
+static int coop_packets(int nblk) { return nblk > 1 ? 64 * nblk + 3 * kCoopCopies : 0; }
+
+// (float)sqrt(1 / m): the reciprocal square root of m's leading part, and one Newton step with m in
+// full (1 - m y^2 to 1e-14), where the FP64 division and root take 1200 cycles.
+__device__ __forceinline__ float oc_rsqrt(double m) {
+    if (!(m > 1e-30 && m < 1e30)) return (float)sqrt(1.0 / m);
+    const float h = (float)m, l = (float)(m - (double)h), y = rsqrtf(h), p = __fmul_rn(y, y);
+    float e = __fmaf_rn(-h, p, 1.0f);
+    e = __fmaf_rn(-h, __fmaf_rn(y, y, -p), e);
+    e = __fmaf_rn(-l, p, e);
+    return __fmaf_rn(0.5f * y, e, y);
+}
+// Bisection's test of an interval; the division only where the answer is not clear without.
+__device__ __forceinline__ bool oc_stop(double lo, double hi, const OcParams &P) {
+    const double d = hi - lo, s = lo + hi + P.tol_eps;
+    if (d > 1.000001 * P.tol * s && s > 0.0) return false;
+    return d / s < P.tol;
+}
 
 // p, q and w d of an element; base gains w a.
 __device__ __forceinline__ float3 oc_line(float xe, float dce, float we, bool pre, const OcParams &P, float sfloor,
@@ -704,16 +727,17 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
                    const uint8_t *__restrict__ pres, const float *__restrict__ w, uint4 *box, OcScalars *sc,
                    float *xnew, int keep, unsigned polls) {
     extern __shared__ float coop_sh[];
-    float *s_part = coop_sh, *kp = s_part + (kOcNodes + 1) * kCoopRow, *kq = kp + keep, *kw = kq + keep;
-    __shared__ float s_sq[kOcNodes];
-    __shared__ int s_stop[kOcNodes];
-    __shared__ double s_mid[kOcNodes];
-    __shared__ double s_tot[kOcNodes + 1];
+    float *s_part = coop_sh, *kp = s_part + kCoopSums / sizeof(float), *kq = kp + keep, *kw = kq + keep;
+    __shared__ float s_sq[kCoopNodes + 1];
+    __shared__ int s_stop[kCoopNodes + 1];
+    __shared__ double s_mid[kCoopNodes + 1];
+    __shared__ double s_tot[kCoopNodes + 1];
     __shared__ double s_lim[3];  // l1, l2, lfinal
     __shared__ int s_steps, s_done, s_ok;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int half = tid >> 8, ht = tid & (kCoopThreads / 2 - 1);
     const int nblk = gridDim.x, bid = blockIdx.x;
-    uint4 *answer = box + 32 * nblk;
+    uint4 *answer = box + 64 * nblk;
     if (tid == 0) {
         s_lim[0] = sc->l1;
         s_lim[1] = sc->l2;
@@ -721,25 +745,26 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
         s_steps = sc->steps;
         s_done = sc->done;
         s_ok = 1;
+        s_sq[kCoopNodes] = 0.0f;
     }
     const float sfloor = sqrtf(P.sqrt_floor);
     const double target = P.volfrac * (double)n - sc->npres;  // vol > volfrac <=> sum > target
-    const int64_t first = (int64_t)bid * kCoopThreads + tid, stride = (int64_t)nblk * kCoopThreads;
-    // the kept elements of this thread: only it reads them back
-    float kept = 0.0f;
-    int nk = 0;
-    for (int64_t e = first; e < n && nk * kCoopThreads < keep; e += stride, ++nk) {
-        const float3 l = oc_line(x[e], dc[e], w[e], pres && pres[e], P, sfloor, kept);
-        kp[nk * kCoopThreads + tid] = l.x;
-        kq[nk * kCoopThreads + tid] = l.y;
-        kw[nk * kCoopThreads + tid] = l.z;
+    const int64_t block0 = (int64_t)bid * kCoopThreads, stride = (int64_t)nblk * kCoopThreads;
+    float kept = 0.0f;  // w a of the kept elements
+    for (int k = tid; k < keep; k += kCoopThreads) {
+        const int64_t e = block0 + tid + (int64_t)(k / kCoopThreads) * stride;
+        float3 l = make_float3(0.0f, 0.0f, 0.0f);
+        if (e < n) l = oc_line(x[e], dc[e], w[e], pres && pres[e], P, sfloor, kept);
+        kp[k] = l.x;
+        kq[k] = l.y;
+        kw[k] = l.z;
     }
     __syncthreads();
     // Rounds have two shapes. While l1 is still 0 the bisection's midpoints are l2/2, l2/4, ...
     // for as long as every volume stays at or below the target (each step sets l2 = mid); a
-    // chain round evaluates the next kOcNodes midpoints of that all-left path, formed exactly
+    // chain round evaluates the next kCoopNodes midpoints of that all-left path, formed exactly
     // as bisection forms them (0.5 (hi + 0)), and ends at the first step that goes right. Once
-    // l1 > 0, tree rounds evaluate the full kOcLevels-level tree. Each round advances the
+    // l1 > 0, tree rounds evaluate the full kCoopLevels-level tree. Each round advances the
     // bisection by at least one step, so max_bisect rounds bound the loop.
     for (int round = 0; round < P.max_bisect; ++round) {
         // block-uniform: written before the last __syncthreads. Through a shuffle, so that the compiler
@@ -747,14 +772,15 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
         if (__shfl_sync(0xffffffffu, (int)(s_done != 0 || s_ok == 0), 0)) break;
         const bool chain = s_lim[0] == 0.0;
         const unsigned ep = (unsigned)round + 1;
-        if (warp < 2 && lane < kOcNodes) {
+        if (tid < 128 && (tid & 63) < kCoopNodes) {  // the midpoints by two warps, the stop tests by two
+            const int node = tid & 63;
             double lo = s_lim[0], hi = s_lim[1];
             if (chain) {
                 // halvings 0.5 (hi + 0) of the all-left path: exact, so the same bits as that
                 // loop of dependent FP64 operations (l2 <= 1e9 stays far above the subnormals)
-                hi = ldexp(hi, -lane);
+                hi = ldexp(hi, -node);
             } else {
-                const int path = lane + 1, depth = 31 - __clz(path);
+                const int path = node + 1, depth = 31 - __clz(path);
                 for (int i = depth - 1; i >= 0; --i) {
                     const double m = 0.5 * (hi + lo);
                     if ((path >> i) & 1)
@@ -763,49 +789,57 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
                         hi = m;
                 }
             }
-            if (warp == 0) {
+            if (tid < 64) {
                 const double m = 0.5 * (hi + lo);
-                s_mid[lane] = m;
-                s_sq[lane] = (float)sqrt(1.0 / m);
+                s_mid[node] = m;
+                s_sq[node] = oc_rsqrt(m);
             } else {
-                s_stop[lane] = (hi - lo) / (lo + hi + P.tol_eps) < P.tol;
+                s_stop[node] = oc_stop(lo, hi, P);
             }
         }
         __syncthreads();
-        float sq[kOcNodes], v[kOcNodes], base = kept;
+        float sq[32], v[32], base = kept;
 #pragma unroll
-        for (int t = 0; t < kOcNodes; ++t) {
-            sq[t] = s_sq[t];
+        for (int t = 0; t < 32; ++t) {
+            sq[t] = s_sq[32 * half + t];
             v[t] = 0.0f;
         }
         auto trials = [&](float p, float q, float wd) {
 #pragma unroll
-            for (int t = 0; t < kOcNodes; ++t) v[t] = fmaf(wd, __saturatef(fmaf(p, sq[t], q)), v[t]);
+            for (int t = 0; t < 32; ++t) {
+                float y;
+                asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(p), "f"(sq[t]), "f"(q));
+                v[t] = fmaf(wd, y, v[t]);
+            }
         };
 #pragma unroll 2
-        for (int k = 0; k < nk; ++k)
-            trials(kp[k * kCoopThreads + tid], kq[k * kCoopThreads + tid], kw[k * kCoopThreads + tid]);
-        for (int64_t e = first + (int64_t)nk * stride; e < n; e += stride) {
-            const float3 l = oc_line(x[e], dc[e], w[e], pres && pres[e], P, sfloor, base);
-            trials(l.x, l.y, l.z);
-        }
+        for (int k = ht; k < keep; k += kCoopThreads / 2) trials(kp[k], kq[k], kw[k]);
+        for (int64_t e0 = block0 + (int64_t)(keep / kCoopThreads) * stride + ht; e0 < n; e0 += stride)
+            for (int64_t e = e0; e < n && e <= e0 + kCoopThreads / 2; e += kCoopThreads / 2) {
+                float a = 0.0f;
+                const float3 l = oc_line(x[e], dc[e], w[e], pres && pres[e], P, sfloor, a);
+                trials(l.x, l.y, l.z);
+                if (half == 0) base += a;
+            }
 #pragma unroll
-        for (int t = 0; t < kOcNodes; ++t) s_part[t * kCoopRow + tid] = v[t];
-        s_part[kOcNodes * kCoopRow + tid] = base;
+        for (int t = 0; t < 32; ++t)
+            if (32 * half + t < kCoopNodes) s_part[(32 * half + t) * kCoopRow + ht] = v[t];
+        s_part[kCoopNodes * kCoopRow + tid] = base;
         __syncthreads();
-        // block sums: node t summed by 16 lanes (columns sub, sub + 16, ...), then across those lanes; the
+        // block sums: node t summed by 8 lanes (columns sub, sub + 8, ...), then across those lanes; the
         // sums' errors carried; every sum in a fixed order
-        const int t = tid >> 4, sub = tid & 15;
+        const int t = tid >> 3, sub = tid & 7, columns = t == kCoopNodes ? kCoopThreads : kCoopThreads / 2;
         ddv a{0.0f, 0.0f};
 #pragma unroll 8
-        for (int j = sub; j < kCoopThreads; j += 16) {
+        for (int j = sub; j < columns; j += 8) {
             float e;
             two_sum(a.h, s_part[t * kCoopRow + j], a.h, e);
             a.l += e;
         }
+        __syncwarp();
         auto across = [&]() {
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1)
+            for (int o = 4; o > 0; o >>= 1)
                 a = dd_add(a, ddv{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)});
         };
         across();
@@ -813,32 +847,31 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
         if (nblk > 1) {
             if (sub == 0) st_packet(box + t * nblk + bid, __float_as_uint(a.h), __float_as_uint(a.l), 0, ep);
             if (bid == 0) {
-                float2 pv[kCoopPer];
-                unsigned need = 0;
+                // ten packets polled together, one round trip per sweep
+                a = ddv{0.0f, 0.0f};
+#pragma unroll 1
+                for (int m0 = sub; m0 < nblk && ok; m0 += 8 * kCoopPoll) {
+                    uint4 u[kCoopPoll];
 #pragma unroll
-                for (int m = 0; m < kCoopPer; ++m) {
-                    pv[m] = make_float2(0.0f, 0.0f);
-                    if (sub + 16 * m < nblk) need |= 1u << m;
-                }
-                for (unsigned sweep = 0; need != 0; ++sweep) {
-                    if (sweep >= polls) {
-                        ok = false;
-                        break;
-                    }
+                    for (int m = 0; m < kCoopPoll; ++m)
+                        u[m] = make_uint4(0, 0, 0, m0 + 8 * m < nblk ? ep - 1 : ep);
+                    bool all;
+                    unsigned sweep = 0;
+#pragma unroll 1
+                    do {
+                        all = true;
 #pragma unroll
-                    for (int m = 0; m < kCoopPer; ++m)
-                        if ((need >> m) & 1u) {
-                            const uint4 u = ld_packet(box + t * nblk + sub + 16 * m);
-                            if (u.w == ep) {
-                                pv[m] = make_float2(__uint_as_float(u.x), __uint_as_float(u.y));
-                                need &= ~(1u << m);
-                            }
-                        }
+                        for (int m = 0; m < kCoopPoll; ++m)
+                            if (u[m].w != ep) u[m] = ld_packet(box + t * nblk + m0 + 8 * m);
+#pragma unroll
+                        for (int m = 0; m < kCoopPoll; ++m) all = all && u[m].w == ep;
+                    } while (!all && ++sweep < polls);
+                    ok = all;
+#pragma unroll
+                    for (int m = 0; m < kCoopPoll; ++m)
+                        a = dd_add(a, ddv{__uint_as_float(u[m].x), __uint_as_float(u[m].y)});
                 }
                 __syncwarp();
-                a = ddv{pv[0].x, pv[0].y};
-#pragma unroll
-                for (int m = 1; m < kCoopPer; ++m) a = dd_add(a, ddv{pv[m].x, pv[m].y});
                 across();
             } else if (tid < 3) {
                 uint4 u = ld_packet(answer + 3 * (bid & (kCoopCopies - 1)) + tid);
@@ -861,32 +894,70 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
             if (sub == 0) s_tot[t] = dd_value(a);
             __syncthreads();
             if (warp == 0) {  // bisection's tests along the chain or the tree (oc_multi_kernel's walk)
-                const bool node = lane < kOcNodes;
-                const unsigned right = __ballot_sync(0xffffffffu, node && s_tot[node ? lane : 0] + s_tot[kOcNodes] > target);
-                const unsigned stop = __ballot_sync(0xffffffffu, node && s_stop[node ? lane : 0]);
-                int steps = s_steps, done = 0, at = 0, n1 = -1, n2 = -1, nf = 0;
-                for (int lvl = 0; lvl < (chain ? kOcNodes : kOcLevels); ++lvl) {
-                    nf = at;
-                    ++steps;
-                    if ((stop >> at) & 1u) {
-                        done = 1;
-                        break;
+                unsigned long long right = 0, stop = 0;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int node = lane + 32 * h;
+                    const bool is = node < kCoopNodes;
+                    const unsigned r = __ballot_sync(0xffffffffu, is && s_tot[node] + s_tot[kCoopNodes] > target);
+                    const unsigned st = __ballot_sync(0xffffffffu, is && s_stop[node]);
+                    right |= (unsigned long long)r << (32 * h);
+                    stop |= (unsigned long long)st << (32 * h);
+                }
+                // the nodes whose midpoints become l1, l2 and lfinal (-1: none)
+                int steps = s_steps, done = 0, n1 = -1, n2 = -1, nf;
+                if (chain) {
+                    // left as far as the first stop or step to the right (tree rounds from there) goes
+                    const int event = __ffsll((long long)(stop | right)) - 1;
+                    const int left = event < 0 ? kCoopNodes : event, room = P.max_bisect - steps;
+                    if (event >= 0 && left < room) {
+                        steps += left + 1;
+                        nf = left;
+                        n2 = left - 1;
+                        if ((stop >> left) & 1u) {
+                            done = 1;
+                        } else {
+                            n1 = left;
+                            done = steps >= P.max_bisect;
+                        }
+                    } else {
+                        const int took = left < room ? left : room;
+                        steps += took;
+                        nf = n2 = took - 1;
+                        done = steps >= P.max_bisect;
                     }
-                    const bool r = (right >> at) & 1u;
-                    if (r)
-                        n1 = at;
-                    else
-                        n2 = at;
-                    at = r ? 2 * at + 2 : (chain ? at + 1 : 2 * at + 1);
-                    if (steps >= P.max_bisect) {
-                        done = 1;
-                        break;
+                } else {
+                    int at = 0;
+                    for (int lvl = 0; lvl < kCoopLevels; ++lvl) {
+                        nf = at;
+                        ++steps;
+                        if ((stop >> at) & 1u) {
+                            done = 1;
+                            break;
+                        }
+                        const bool r = (right >> at) & 1u;
+                        if (r)
+                            n1 = at;
+                        else
+                            n2 = at;
+                        at = 2 * at + (r ? 2 : 1);
+                        if (steps >= P.max_bisect) {
+                            done = 1;
+                            break;
+                        }
                     }
-                    if (chain && r) break;  // off the all-left path: tree rounds from here
                 }
                 if (lane < 3) {
                     const int from = lane == 0 ? n1 : (lane == 1 ? n2 : nf);
                     if (from >= 0) s_lim[lane] = s_mid[from];
+                }
+                __syncwarp();
+                // the next step's stop test spares the round that would only find it
+                const double lo = s_lim[0], hi = s_lim[1];
+                if (!done && lo > 0.0 && oc_stop(lo, hi, P)) {
+                    done = 1;
+                    ++steps;
+                    if (lane == 2) s_lim[2] = 0.5 * (hi + lo);
                 }
                 if (lane == 0) {
                     s_steps = steps;
@@ -911,7 +982,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
         sc->done = s_done;
     }
     const float inv_l = (float)(1.0 / s_lim[2]);
-    for (int64_t e = first; e < n; e += stride) xnew[e] = oc_trial(x[e], dc[e], inv_l, P, pres && pres[e]);
+    for (int64_t e = block0 + tid; e < n; e += stride) xnew[e] = oc_trial(x[e], dc[e], inv_l, P, pres && pres[e]);
 }
 
 __global__ void oc_final_kernel(int64_t n, const OcParams P, const float *__restrict__ x,

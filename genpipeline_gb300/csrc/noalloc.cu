@@ -9,10 +9,10 @@
 
 #include "internal.h"
 
-// Scratch of gbsimp_oc_noalloc: 16.1 MiB, enough for GBSIMP_OC_NOALLOC_MAX_ELEMENTS
+// Scratch of gbsimp_oc_noalloc: 16.2 MiB, enough for GBSIMP_OC_NOALLOC_MAX_ELEMENTS
 // elements. It is a module-scope device array: every GPU that loads this library holds it
 // until the process exits, whether or not the entry point is called.
-#define GBS_OC_NOALLOC_BYTES (256 + 2 * (4 * GBSIMP_OC_NOALLOC_MAX_ELEMENTS) + 4 * 4096 * 8)
+#define GBS_OC_NOALLOC_BYTES (256 + 2 * (4 * GBSIMP_OC_NOALLOC_MAX_ELEMENTS) + 4 * 4096 * 8 + 65536)
 static __device__ __align__(256) unsigned char g_oc_noalloc_scratch[GBS_OC_NOALLOC_BYTES];
 
 namespace {

@@ -195,7 +195,7 @@ int gbsimp_oc(gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin,
  * that cannot allocate device memory: a host-language plugin that reaches the GPU only
  * through this C ABI and has no CUDA allocator of its own, or a serving process whose device
  * memory is reserved up front and must not grow per request. Same inputs, outputs and
- * results as gbsimp_oc, but the scratch is a fixed 16.1 MiB device array inside the library
+ * results as gbsimp_oc, but the scratch is a fixed 16.2 MiB device array inside the library
  * (held on every GPU that loads the library until the process exits), so grids above
  * GBSIMP_OC_NOALLOC_MAX_ELEMENTS elements are rejected with GBS_EINVAL. The first call on a
  * device looks up that array's device address (call it with the context's device current);
