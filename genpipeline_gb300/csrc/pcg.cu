@@ -1107,8 +1107,8 @@ struct ApplyProfile {
 
 // ---- the on-chip form (pcg_chip.cu) ---------------------------------------------------------
 // Whenever the grid fits the chip: it is the faster form at every size that does. us per iteration of
-// a solve, streaming in the graph loop -> on the chip: 8x4x4 7.5 -> 2.1, 32x8x8 7.9 -> 4.1, 32^3
-// 8.4 -> 4.4, 48^3 10.7 -> 5.6, 95x47x33 11.9 -> 6.7, 64^3 (about the most it holds) 13.9 -> 10.1.
+// a solve, streaming in the graph loop -> on the chip: 8x4x4 7.5 -> 1.7, 32x8x8 7.9 -> 3.9, 32^3
+// 8.4 -> 4.2, 48^3 10.7 -> 5.3, 95x47x33 11.9 -> 6.7, 64^3 (about the most it holds) 13.9 -> 8.9.
 static inline bool chip_ok(const gbsimp_ctx *ctx, const ChipItem &it) {
     return use_modal(ctx, it.nz) && chip_min_blocks(ctx, it) > 0;
 }

@@ -7,9 +7,8 @@
 // (a serial march over node planes, each waiting for its copies) and 13.9 us with the fold of
 // the partial sums and the launch gap, where its arithmetic takes 1.4 us of the SMs' FP32 rate.
 // 152 SMs hold 34 MB of shared memory and 39 MB of registers; the PCG state of 64^3 is 20 MB.
-// Here an iteration of 32^3 takes 4.4 us (streaming 8.4): march 1.5, exchange 2.5, sums 0.3,
-// update 0.2. One of 64^3 takes 10.1: its kernel (six places per thread) has about 55 KB of loop
-// code, more than the instruction cache holds, and its exchange takes twice as long for it.
+// Here an iteration of 32^3 takes 4.1 us (streaming 8.4): march 1.4, exchange 2.2, sums 0.3,
+// update 0.2; one of 64^3 8.9, of which 0.8 is its kernel's code not fitting the instruction cache.
 // Split. The elements are cut into Px x Py x Pz boxes, one per CTA. A CTA holds all nodes of its
 // box, so nodes on a face between boxes are held by both. The box's K u is a partial sum there;
 // per iteration the CTAs exchange those partials (a node's 12 bytes) and three sums, and every
@@ -33,7 +32,10 @@
 // packed into warps) and marches two slabs of it at once in the lanes of packed FP32x2
 // instructions, carrying the (y, z)-transformed node plane and the cx = 1 half to the next step.
 // The cz = 1 halves reach the lane above by a shuffle; the cy = 0 and cy = 1 sums go to two
-// arrays (W0, W1) with one writer each, so the march needs no block barrier.
+// arrays (W0, W1) with one writer each, so the march needs no block barrier. The slabs' end planes
+// are joined behind the march by the warps that have no sums to send: in the march's last step it
+// took 0.2 us longer (two or three sets of loads, adds and stores at the end of its serial chain) and 4 KB
+// of code.
 #include <math.h>
 #include <string.h>
 
@@ -173,19 +175,6 @@ __device__ __forceinline__ void chip_element(float2 (&v)[8][3], float2 E, const 
     for (int c = 0; c < 3; ++c) v[0][c] = make_float2(0.0f, 0.0f);
 }
 
-// v.x joins word nx + o, v.y word ny + o (when there is one); v takes the sums.
-__device__ __forceinline__ void chip_join(float *f, int nx, int ny, int o, float2 &v) {
-    v.x += f[nx + o];
-    f[nx + o] = v.x;
-    if (ny >= 0) {
-        v.y += f[ny + o];
-        f[ny + o] = v.y;
-    }
-}
-
-// A block barrier that warps reach from different places.
-__device__ __forceinline__ void bar_sync_all() { asm volatile("bar.sync 1, %0;" ::"n"(kChipNT) : "memory"); }
-
 // (y, z) forward butterflies of one node plane's four corners (b = cy * 2 + cz).
 __device__ __forceinline__ void chip_yz_forward(float2 (&q)[4][3]) {
 #pragma unroll
@@ -270,6 +259,12 @@ __global__ void __launch_bounds__(kChipNT, 1)
     };
     // ---- the vectors: thread tid holds node pairs tid, tid + 256, ... ---------------------------
     float2 r[Q][3], s[Q][3], p[Q][3];
+    // The widest kernel's loop code outgrows the instruction cache (at 64^3 a warp waited for code 18 % of
+    // the time): it takes the shorter forms of two parts, which the others are slower with (64^3 9.8 ->
+    // 8.9 us, 60^3 7.6 -> 8.1 with both): two packets polled together instead of four, and x updated in
+    // every iteration instead of in every other, for two.
+    constexpr bool kTight = Q > 5;
+    constexpr int kPoll = kTight ? 2 : 4;
     unsigned own = 0;  // bit 2 q + h: counts in this CTA's sums (one of a shared node's holders counts it)
     const bool fresh = I.fresh != 0;
     const volatile PcgScalars *vsc = sc;
@@ -447,6 +442,23 @@ __global__ void __launch_bounds__(kChipNT, 1)
         }
         return c;
     };
+    // The halves of w at the slabs' ends: a slab's last plane and the next slab's first are the same
+    // nodes, and both copies take the sum (by all warps but the first, which has the sums to send).
+    auto join = [&]() {
+        float *f0 = (float *)W0, *f1 = (float *)W1;
+#pragma unroll 1
+        for (int e = tid - 32; e < (2 * g.G - 1) * SY; e += kChipNT - 32) {
+            const int slab = e / SY, jk = e - slab * SY, next = slab + 1;
+            const int hl = slab >= g.G, hn = next >= g.G;
+            const int a = word_of((((slab - hl * g.G) * NP + L) * SY + jk) << 1 | hl, 0);
+            const int b = word_of(((next - hn * g.G) * NP * SY + jk) << 1 | hn, 0);
+#pragma unroll
+            for (int c = 0; c < 6; c += 2) {
+                f0[a + c] = f0[b + c] = f0[a + c] + f0[b + c];
+                f1[a + c] = f1[b + c] = f1[a + c] + f1[b + c];
+            }
+        }
+    };
     const int it_end = budget > 0 ? it + budget : 0x7fffffff;
 
     while (!done && (first || it < it_end)) {
@@ -456,7 +468,7 @@ __global__ void __launch_bounds__(kChipNT, 1)
         // x takes two steps at once, every other iteration: x_{i+1} = x_{i-1} +
         // (alpha_{i-1} + alpha_i beta_i) p_{i-1} + alpha_i u_i
         const float c1 = fmaf(al, be, alpha_prev);
-        const float2 c12 = make_float2(c1, c1);
+        const float2 c12 = make_float2(c1, c1), ap2 = make_float2(alpha_prev, alpha_prev);
         float2 g_ru = make_float2(0.0f, 0.0f), g_rr = g_ru;
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
@@ -467,13 +479,14 @@ __global__ void __launch_bounds__(kChipNT, 1)
             for (int c = 0; c < 3; ++c) {
                 w[c] = add2(W0[n3 + c], W1[n3 + c]);
                 d[c] = Dv[n3 + c];
-                if (two) x[c] = Xs[n3 + c];
+                if (kTight || two) x[c] = Xs[n3 + c];
             }
             float2 ru = make_float2(0.0f, 0.0f), rr = ru;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float2 uo = __fmul2_rn(d[c], r[q][c]);
-                if (two) Xs[n3 + c] = __ffma2_rn(c12, p[q][c], __ffma2_rn(al2, uo, x[c]));
+                if (kTight) Xs[n3 + c] = __ffma2_rn(ap2, p[q][c], x[c]);
+                else if (two) Xs[n3 + c] = __ffma2_rn(c12, p[q][c], __ffma2_rn(al2, uo, x[c]));
                 s[q][c] = __ffma2_rn(be2, s[q][c], w[c]);
                 p[q][c] = __ffma2_rn(be2, p[q][c], uo);
                 const float2 rn = __ffma2_rn(na2, s[q][c], r[q][c]);
@@ -531,8 +544,6 @@ __global__ void __launch_bounds__(kChipNT, 1)
                             g1[b][c] = add2(v[b][c], v[4 + b][c]);
                         }
                 } else {
-                    // the first planes of the other pairs' slabs are stored by their warps
-                    if (g.G > 1) bar_sync_all();
 #pragma unroll
                     for (int b = 0; b < 4; ++b)
 #pragma unroll
@@ -550,23 +561,6 @@ __global__ void __launch_bounds__(kChipNT, 1)
                 if (col_ok) {
                     const int n = base + 3 * SY * t;
                     float2 *w0 = W0 + n, *w1 = W1 + n + 3 * SZ;
-                    if (t == L) {
-                        // a slab's last plane: its half joins the next slab's first one, and both copies
-                        // take the sum
-                        const int here = base - 3 * gp * NP * SY;
-                        const int nx = gp + 1 < g.G ? 2 * (base + 3 * NP * SY) : 2 * here + 1;
-                        const int ny = gp + 1 < g.G ? 2 * (base + 3 * NP * SY) + 1 : -1;
-                        float *f0 = (float *)W0, *f1 = (float *)W1 + 6 * SZ;
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            chip_join(f0, nx, ny, 2 * c, h[0][c]);
-                            chip_join(f1, nx, ny, 2 * c, h[2][c]);
-                            if (top) {
-                                chip_join(f0, nx, ny, 6 + 2 * c, h[1][c]);
-                                chip_join(f1, nx, ny, 6 + 2 * c, h[3][c]);
-                            }
-                        }
-                    }
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
                         w0[c] = h[0][c];
@@ -580,8 +574,6 @@ __global__ void __launch_bounds__(kChipNT, 1)
                         }
                 }
             }
-        } else if (g.G > 1) {
-            bar_sync_all();
         }
 
         // ---- sums, exchange ------------------------------------------------------------------------
@@ -607,7 +599,10 @@ __global__ void __launch_bounds__(kChipNT, 1)
                     st_packet(mail + 2 * bid + 1, __float_as_uint(v3[1].l), __float_as_uint(v3[2].h),
                               __float_as_uint(v3[2].l), ep);
                 }
+            } else {
+                join();
             }
+            __syncthreads();
             const float *f0 = (const float *)W0, *f1 = (const float *)W1;
 #pragma unroll 2
             for (int e = tid; e < ns; e += kChipNT) {
@@ -672,11 +667,11 @@ __global__ void __launch_bounds__(kChipNT, 1)
             // sent by one thread and settled by others.
             __syncthreads();
 #pragma unroll 1
-            for (int e0 = tid; ok && e0 < ni; e0 += 4 * kChipNT) {
-                uint2 at[4];
-                uint4 v[4];
+            for (int e0 = tid; ok && e0 < ni; e0 += kPoll * kChipNT) {
+                uint2 at[kPoll];
+                uint4 v[kPoll];
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
+                for (int m = 0; m < kPoll; ++m) {
                     const int e = e0 + m * kChipNT;
                     at[m] = item[e < ni ? e : e0];
                     v[m].w = e < ni ? ep - 1 : ep;
@@ -687,14 +682,14 @@ __global__ void __launch_bounds__(kChipNT, 1)
                 do {
                     all = true;
 #pragma unroll
-                    for (int m = 0; m < 4; ++m)
+                    for (int m = 0; m < kPoll; ++m)
                         if (v[m].w != ep) v[m] = ld_packet(xp + (int)at[m].x);
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) all = all && v[m].w == ep;
+                    for (int m = 0; m < kPoll; ++m) all = all && v[m].w == ep;
                 } while (!all && ++sweep < polls);
                 ok = all;
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
+                for (int m = 0; m < kPoll; ++m) {
                     if (e0 + m * kChipNT >= ni) continue;
                     const float x = __uint_as_float(v[m].x), y = __uint_as_float(v[m].y), z = __uint_as_float(v[m].z);
                     if (at[m].y >> 31) {
@@ -744,6 +739,8 @@ __global__ void __launch_bounds__(kChipNT, 1)
             if (warp == 0) {
                 box_sums(red, v3);
                 step(v3);
+            } else {
+                join();
             }
             __syncthreads();
         }
@@ -767,7 +764,7 @@ __global__ void __launch_bounds__(kChipNT, 1)
     }
     // ---- the iterate out; a paused solve's state too -------------------------------------------
     // x owes the last iteration's step when that one did not update it
-    const float owed = two ? alpha_prev : 0.0f;
+    const float owed = kTight || two ? alpha_prev : 0.0f;
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int n = tid + kChipNT * q;
@@ -813,15 +810,14 @@ __global__ void __launch_bounds__(kChipNT, 1)
 // Modelled SM cycles of one iteration of a box, fitted to clock counts of its phases over boxes of
 // 2x8x8 to 16x8x16 elements (within 10 %): the march's steps, dearer with a second warp on a
 // scheduler and with several slabs of rows longer than four (their planes meet in shared memory's
-// banks); the update of q places per thread, dearer in the widest kernel, whose iteration outgrows the
-// instruction cache; the block's sums; the exchange.
+// banks); the update of q places per thread; the block's sums; the exchange; and what the widest
+// kernel, whose iteration outgrows the instruction cache, takes longer.
 static double chip_cost(int ex, int ez, int q, int warps, int G, int nblk, int items) {
     const int L = (ex + 2 * G - 1) / (2 * G);
     double c = 1560.0 + L * (650.0 + 55.0 * std::min(warps, 4) + (warps > 4 ? 370.0 : 0.0));
     if (G > 1) c += 100.0 + (ez > 4 ? 100.0 * warps * L : 0.0);
-    c += 700.0 + (q > 4 ? 530.0 : 320.0) * q;
-    if (nblk == 1) return c + 630.0;
-    return c + 4500.0 + 1.6 * items + (q > 4 ? 3000.0 : 0.0);
+    c += 700.0 + 320.0 * q + (q > 5 ? 2500.0 : 0.0);
+    return c + (nblk > 1 ? 4500.0 + 1.6 * items : 630.0);
 }
 
 // Every way to cut the grid into at most max_blocks boxes; f(geom, nblk, cost) for each that fits.
@@ -856,9 +852,10 @@ static void chip_each(int nx, int ny, int nz, int max_blocks, F &&f) {
 }
 
 using ChipKernel = void (*)(const ModalK, unsigned, int, const ChipTable);
-// Places per thread of the largest box, rounded up to a kernel's: 95x47x33 (four) takes 7.3 us per
-// iteration in its own kernel, 11.4 in the one for six; one for three measured no better than four's.
-static const ChipKernel chip_kern[4] = {pcg_chip_kernel<1>, pcg_chip_kernel<2>, pcg_chip_kernel<4>,
+// Places per thread of the largest box, rounded up to a kernel's: 95x47x33 (four) took 7.3 us per
+// iteration in its own kernel and 11.4 in the one for six, 60^3 (five) 7.6 and 8.0; one for three measured
+// no better than four's.
+static const ChipKernel chip_kern[5] = {pcg_chip_kernel<1>, pcg_chip_kernel<2>, pcg_chip_kernel<4>, pcg_chip_kernel<5>,
                                         pcg_chip_kernel<kChipQ>};
 
 // Sets the kernels' shared-memory limit once per device; false without cooperative launches.
@@ -985,7 +982,7 @@ int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cu
         smem = std::max(smem, chip_smem(D.g.G * (L + 1) * D.g.NYm * D.g.NZm, L * D.g.G * (D.g.NYm - 1) * (D.g.NZm - 1),
                                         chip_shared(ex + 2 * D.g.G, D.g.NYm, D.g.NZm, D.g.Px, D.g.Py, D.g.Pz, true)));
     }
-    const int v = q <= 1 ? 0 : (q <= 2 ? 1 : (q <= 4 ? 2 : 3));
+    const int v = q <= 1 ? 0 : (q <= 2 ? 1 : (q <= 4 ? 2 : (q <= 5 ? 3 : 4)));
     for (int i = 0; i < n; ++i) {
         // no packet of an earlier launch may carry an epoch of this one
         if (T.d[i].nblk > 1)
