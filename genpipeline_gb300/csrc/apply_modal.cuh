@@ -52,15 +52,15 @@ template <int NT>
 __host__ __device__ constexpr int modal_layout_r(int R) { return (3 * R + 6) / 4 <= 2 * NT ? modal_r2<NT>() : R; }
 
 // Shared memory of the modal kernel for a given z extent (NT = 256, EPT = 2): four operand
-// planes and the raw bulk-copy buffers (one per staged vector: p for the plain apply; r, w,
-// s, 1/diag, p, x for the PCG modes), modal_rw floats each, two planes of element moduli, and
+// planes and the raw bulk-copy buffers (one per staged vector: r, w, s, 1/diag, p, x), modal_rw
+// floats each, two planes of element moduli, and
 // two copies (by step parity) of the y-direction slots (3 floats per element) and of the
 // warp-boundary contributions (6 floats per warp and lane).
 template <int NT, int EPT>
-inline size_t modal_smem_bytes(int nz, bool cg) {
+inline size_t modal_smem_bytes(int nz) {
     const int NE = NT * EPT, H = nz + 2, R = modal_layout_r<NT>(NE + H);
     const size_t RW = (size_t)modal_rw(R);
-    return 4 * RW * sizeof(float) + (cg ? 6 : 1) * RW * sizeof(float) + (2 + 6) * (size_t)NT * sizeof(float2) +
+    return 4 * RW * sizeof(float) + 6 * RW * sizeof(float) + (2 + 6) * (size_t)NT * sizeof(float2) +
            2 * (size_t)(NT / 32) * 6 * sizeof(float2);
 }
 
@@ -125,28 +125,8 @@ __device__ __forceinline__ float2 shfl_up2(float2 v) {
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
 
-// Two elements at once: corners v[b][c] (b = cx*4 + cy*2 + cz) -> E (Ke p_e)_b,c for each
-// lane. The operations and their order per lane are those of the scalar form: forward
-// butterflies, r = Km q (each row summed in column order), r *= E, inverse butterflies.
-// With XONLY the inverse stops after its x stage: v[b] (b < 4) is then the (y, z)-modal cx = 0
-// half and v[4 + b] the cx = 1 half, to be summed per node plane before yz_inverse2.
-template <bool XONLY>
-__device__ __forceinline__ void modal_element2(float2 (&v)[8][3], float2 E, const ModalK &km) {
-    // forward Walsh-Hadamard per component: (u0, u1) -> (u0 + u1, u1 - u0)
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const int bit = 1 << d;
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            if (b & bit) continue;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float2 u0 = v[b][c], u1 = v[b | bit][c];
-                v[b][c] = add2(u0, u1);
-                v[b | bit][c] = sub2(u1, u0);
-            }
-        }
-    }
+// The modes of two elements, in place: q -> E Km q.
+__device__ __forceinline__ void modal_rows2(float2 (&v)[8][3], float2 E, const ModalK &km) {
     // r = E Km q, one block at a time, in place (mode 0, the translations, has no entries)
 #pragma unroll
     for (int bk = 0; bk < kModalBlocks; ++bk) {
@@ -173,21 +153,39 @@ __device__ __forceinline__ void modal_element2(float2 (&v)[8][3], float2 E, cons
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) v[0][c] = make_float2(0.0f, 0.0f);
-    // inverse: (r0, r1) -> (r0 - r1, r0 + r1) along each axis (x first; the stages commute)
+}
+
+// Two elements at once: corners v[b][c] (b = cx*4 + cy*2 + cz) -> E (Ke p_e)_b,c for each
+// lane. The operations and their order per lane are those of the scalar form: forward
+// butterflies, r = Km q (each row summed in column order), r *= E, inverse butterflies, of which
+// only the x stage runs here: v[b] (b < 4) is then the (y, z)-modal cx = 0 half and v[4 + b] the
+// cx = 1 half, to be summed per node plane before yz_inverse2.
+__device__ __forceinline__ void modal_element2(float2 (&v)[8][3], float2 E, const ModalK &km) {
+    // forward Walsh-Hadamard per component: (u0, u1) -> (u0 + u1, u1 - u0)
 #pragma unroll
-    for (int dd = 0; dd < (XONLY ? 1 : 3); ++dd) {
-        const int bit = 4 >> dd;
+    for (int d = 0; d < 3; ++d) {
+        const int bit = 1 << d;
 #pragma unroll
         for (int b = 0; b < 8; ++b) {
             if (b & bit) continue;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const float2 r0 = v[b][c], r1 = v[b | bit][c];
-                v[b][c] = sub2(r0, r1);
-                v[b | bit][c] = add2(r0, r1);
+                const float2 u0 = v[b][c], u1 = v[b | bit][c];
+                v[b][c] = add2(u0, u1);
+                v[b | bit][c] = sub2(u1, u0);
             }
         }
     }
+    modal_rows2(v, E, km);
+    // inverse along x: (r0, r1) -> (r0 - r1, r0 + r1)
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 r0 = v[b][c], r1 = v[4 + b][c];
+            v[b][c] = sub2(r0, r1);
+            v[4 + b][c] = add2(r0, r1);
+        }
 }
 
 // The (y, z) stages of the inverse transform on one node plane's four corners
@@ -238,15 +236,14 @@ __device__ __forceinline__ float ld_vec(const float *p) {
     return *p;
 }
 
-// One sliding-window pass of a CTA over its (flat tile, x segment): y = D K D p on the owned
-// nodes (PLAIN; x = densities), or one PCG iteration with y = w_{i+1} (CG modes; x = the
-// element moduli E(x_e), computed once per solve). sums[] receives this
-// thread's FP32 shares of r.u, w.u and r.r (CG modes). Every node vector must be 16-byte
+// One sliding-window pass of a CTA over its (flat tile, x segment): one PCG iteration with
+// y = w_{i+1} on the owned nodes; x = the element moduli E(x_e), computed once per solve. sums[]
+// receives this thread's FP32 shares of r.u, w.u and r.r. Every node vector must be 16-byte
 // aligned. pre(alpha, beta, alpha_prev) runs once the first plane's copies are in flight (the
 // step's scalars can be formed meanwhile); when it returns false the pass stops there
 // (returns false).
 //
-// Segments. PLAIN and CG_FUSED: segment s owns node planes [xs, xe) of nx + 1 and also
+// Segments. CG_FUSED: segment s owns node planes [xs, xe) of nx + 1 and also
 // computes element plane xs - 1 (a halo step) so that every owned node sums all its elements.
 // CG: segment s computes element planes [xs, xe) of nx, owns node planes [xs, xe) (the last
 // segment also node plane nx) and outputs node planes xs..xe. Node plane xs of s > 0 and node
@@ -256,17 +253,14 @@ __device__ __forceinline__ float ld_vec(const float *p) {
 // and the w.u shares add up the same way. That saves the halo step's element work and one
 // staged plane per CTA.
 template <int NT, int EPT, int MAXV, int MODE, typename Pre>
-__device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__restrict__ x,
-                                           const float *__restrict__ p, float *__restrict__ y,
-                                           const uint8_t *__restrict__ mask, const Law<float> &law,
+__device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__restrict__ x, float *__restrict__ y,
                                            const ModalK &km, const CgPass &cp, float *smem, int tile, int seg,
                                            float (&sums)[3], Pre &&pre) {
     constexpr int NE = NT * EPT;
-    constexpr bool CG = MODE == MODE_CG || MODE == MODE_CG_FUSED;
-    constexpr int NR = CG ? 6 : 1;  // staged vectors
+    constexpr int NR = 6;  // staged vectors
     static_assert(EPT == 2, "two elements per thread (packed FP32x2)");
     static_assert(NT % 32 == 0, "whole warps");
-    static_assert(MODE == MODE_PLAIN || CG, "modal pass modes: PLAIN, CG, CG_FUSED");
+    static_assert(MODE == MODE_CG || MODE == MODE_CG_FUSED, "modal pass modes: CG, CG_FUSED");
 
     const int nx = G.nx, ny = G.ny, nz = G.nz;
     const int NZ = nz + 1;
@@ -301,7 +295,6 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
     sums[0] = sums[1] = sums[2] = 0.0f;
 
     auto src_of = [&](int a) -> const float * {
-        if (!CG) return p;
         return a == 0 ? cp.r : a == 1 ? cp.w : a == 2 ? cp.sold : a == 3 ? cp.dinv : a == 4 ? cp.p : cp.xu;
     };
     // Word geometry of node plane j: the chunk's words start at W0 = 3 (j S + F0 - H); group f
@@ -336,7 +329,7 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
     // mbarrier phase per plane counts the bytes. Only a group cut by the end of the vectors is
     // copied by its thread with cp.async (zero-filled). The raw buffers are rewritten only after
     // a block barrier that follows every thread's reads of the previous plane.
-    constexpr int NF = CG ? 4 : 1;  // vectors staged over the whole plane
+    constexpr int NF = 4;  // vectors staged over the whole plane
     __shared__ unsigned long long s_bar;
     unsigned bphase = 0;  // phase of the plane being committed
     bool bulk_ok = true;  // false once a wait ran out (then no further waits)
@@ -365,7 +358,7 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
             g0 = max(P.A, (int64_t)0);
             const int64_t g1 = min(P.A + 4 * (int64_t)P.nv, full);
             if (g1 > g0) nfull = (unsigned)(g1 - g0);
-            if (CG && P.own) {  // groups that meet the owned words [olo3, ohi3)
+            if (P.own) {  // groups that meet the owned words [olo3, ohi3)
                 o0 = max(P.A + 4 * (int64_t)((P.olo3 + P.pad) >> 2), (int64_t)0);
                 const int64_t o1 = min(P.A + 4 * (int64_t)((P.ohi3 + P.pad + 3) >> 2), full);
                 if (o1 > o0) nown = (unsigned)(o1 - o0);
@@ -382,7 +375,7 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
         if (nfull)
 #pragma unroll
             for (int a = 0; a < NF; ++a) bulk_prefetch_l2(src_of(a) + g0, 4u * nfull);
-        if (CG && nown)
+        if (nown)
 #pragma unroll
             for (int a = 4; a < 6; ++a)
                 if (a == 4 || cp.xmode) bulk_prefetch_l2(src_of(a) + o0, 4u * nown);
@@ -401,13 +394,12 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
 #pragma unroll
                     for (int a = 0; a < NF; ++a)
                         bulk_copy_g2s(Raw + a * RW + (g0 - P.A), src_of(a) + g0, 4u * nfull, &s_bar);
-                if (CG && nown)
+                if (nown)
 #pragma unroll
                     for (int a = 4; a < 6; ++a)
                         if (a == 4 || cp.xmode)
                             bulk_copy_g2s(Raw + a * RW + (o0 - P.A), src_of(a) + o0, 4u * nown, &s_bar);
-                // the PCG modes (several vectors per plane): the plain apply measured no gain
-                if (CG && j + 1 <= xe) prefetch_plane(j + 1);  // xe: the segment's last staged plane
+                if (j + 1 <= xe) prefetch_plane(j + 1);  // xe: the segment's last staged plane
             }
             // the group cut by the end of the vectors: only the last node plane reaches it
             if (j == nx && full < NW) {
@@ -444,81 +436,65 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
                 const bool own_all = in_all && P.own && cw0 >= P.olo3 && cw0 + 4 <= P.ohi3;
                 const bool own_none = !P.own || cw0 + 4 <= P.olo3 || cw0 >= P.ohi3;
                 float val[4];
-                if (!CG) {
-                    const float4 a4 = *(const float4 *)(Raw + 4 * f);
-                    const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+                const float4 r4 = *(const float4 *)(Raw + 0 * RW + 4 * f);
+                const float4 w4 = *(const float4 *)(Raw + 1 * RW + 4 * f);
+                const float4 s4 = *(const float4 *)(Raw + 2 * RW + 4 * f);
+                const float4 d4 = *(const float4 *)(Raw + 3 * RW + 4 * f);
+                const float rv[4] = {r4.x, r4.y, r4.z, r4.w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
+                const float sv[4] = {s4.x, s4.y, s4.z, s4.w}, dv[4] = {d4.x, d4.y, d4.z, d4.w};
+                float so[4], rno[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    so[k] = fmaf(beta, sv[k], wv[k]);
+                    rno[k] = fmaf(-alpha, so[k], rv[k]);
+                    val[k] = dv[k] * rno[k];
+                }
+                if (own_all) {
+                    const float4 p4 = *(const float4 *)(Raw + 4 * RW + 4 * f);
+                    const float4 x4 = cp.xmode ? *(const float4 *)(Raw + 5 * RW + 4 * f) : make_float4(0, 0, 0, 0);
+                    const float pv[4] = {p4.x, p4.y, p4.z, p4.w}, xv[4] = {x4.x, x4.y, x4.z, x4.w};
+                    float po[4], xo[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float ur = dv[k] * rv[k];  // u_i = M r_i
+                        po[k] = fmaf(beta, pv[k], ur);
+                        xo[k] = cp.xmode == 2 ? fmaf(c1, pv[k], fmaf(alpha, ur, xv[k])) : fmaf(alpha, po[k], xv[k]);
+                        g_ru = fmaf(rno[k], val[k], g_ru);
+                        g_rr = dv[k] != 0.0f ? fmaf(rno[k], rno[k], g_rr) : g_rr;  // free DOFs only
+                    }
+                    *(float4 *)(cp.snew + gw) = make_float4(so[0], so[1], so[2], so[3]);
+                    *(float4 *)(cp.rnew + gw) = make_float4(rno[0], rno[1], rno[2], rno[3]);
+                    *(float4 *)(cp.p + gw) = make_float4(po[0], po[1], po[2], po[3]);
+                    if (cp.xmode) *(float4 *)(cp.xu + gw) = make_float4(xo[0], xo[1], xo[2], xo[3]);
+                } else if (!(in_all && own_none)) {
+                    // edge group: word by word
+                    const bool any_own = !own_none;
+                    float pv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, xv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    if (any_own) {
+                        const float4 p4 = *(const float4 *)(Raw + 4 * RW + 4 * f);
+                        pv[0] = p4.x, pv[1] = p4.y, pv[2] = p4.z, pv[3] = p4.w;
+                        if (cp.xmode) {
+                            const float4 x4 = *(const float4 *)(Raw + 5 * RW + 4 * f);
+                            xv[0] = x4.x, xv[1] = x4.y, xv[2] = x4.z, xv[3] = x4.w;
+                        }
+                    }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const int cw = cw0 + k;
-                        const bool valid = in_all || (P.pv && cw >= P.lo3 && cw < P.hi3);
-                        bool fixed = false;
-                        if (mask && valid) {
-                            const int l = cw / 3;
-                            fixed = (mask[(int64_t)j * S + F0 - H + l] >> (cw - 3 * l)) & 1;
-                        }
-                        val[k] = valid && !fixed ? av[k] : 0.0f;
-                    }
-                } else {
-                    const float4 r4 = *(const float4 *)(Raw + 0 * RW + 4 * f);
-                    const float4 w4 = *(const float4 *)(Raw + 1 * RW + 4 * f);
-                    const float4 s4 = *(const float4 *)(Raw + 2 * RW + 4 * f);
-                    const float4 d4 = *(const float4 *)(Raw + 3 * RW + 4 * f);
-                    const float rv[4] = {r4.x, r4.y, r4.z, r4.w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
-                    const float sv[4] = {s4.x, s4.y, s4.z, s4.w}, dv[4] = {d4.x, d4.y, d4.z, d4.w};
-                    float so[4], rno[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        so[k] = fmaf(beta, sv[k], wv[k]);
-                        rno[k] = fmaf(-alpha, so[k], rv[k]);
-                        val[k] = dv[k] * rno[k];
-                    }
-                    if (own_all) {
-                        const float4 p4 = *(const float4 *)(Raw + 4 * RW + 4 * f);
-                        const float4 x4 = cp.xmode ? *(const float4 *)(Raw + 5 * RW + 4 * f) : make_float4(0, 0, 0, 0);
-                        const float pv[4] = {p4.x, p4.y, p4.z, p4.w}, xv[4] = {x4.x, x4.y, x4.z, x4.w};
-                        float po[4], xo[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const float ur = dv[k] * rv[k];  // u_i = M r_i
-                            po[k] = fmaf(beta, pv[k], ur);
-                            xo[k] = cp.xmode == 2 ? fmaf(c1, pv[k], fmaf(alpha, ur, xv[k])) : fmaf(alpha, po[k], xv[k]);
+                        const bool valid = P.pv && cw >= P.lo3 && cw < P.hi3;
+                        const bool own = valid && any_own && cw >= P.olo3 && cw < P.ohi3;
+                        if (!valid) val[k] = 0.0f;
+                        if (own) {
+                            const float ur = dv[k] * rv[k];
+                            const float po = fmaf(beta, pv[k], ur);
+                            cp.snew[gw + k] = so[k];
+                            cp.rnew[gw + k] = rno[k];
+                            cp.p[gw + k] = po;
+                            if (cp.xmode)
+                                cp.xu[gw + k] =
+                                    cp.xmode == 2 ? fmaf(c1, pv[k], fmaf(alpha, ur, xv[k])) : fmaf(alpha, po, xv[k]);
                             g_ru = fmaf(rno[k], val[k], g_ru);
-                            g_rr = dv[k] != 0.0f ? fmaf(rno[k], rno[k], g_rr) : g_rr;  // free DOFs only
-                        }
-                        *(float4 *)(cp.snew + gw) = make_float4(so[0], so[1], so[2], so[3]);
-                        *(float4 *)(cp.rnew + gw) = make_float4(rno[0], rno[1], rno[2], rno[3]);
-                        *(float4 *)(cp.p + gw) = make_float4(po[0], po[1], po[2], po[3]);
-                        if (cp.xmode) *(float4 *)(cp.xu + gw) = make_float4(xo[0], xo[1], xo[2], xo[3]);
-                    } else if (!(in_all && own_none)) {
-                        // edge group: word by word
-                        const bool any_own = !own_none;
-                        float pv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, xv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                        if (any_own) {
-                            const float4 p4 = *(const float4 *)(Raw + 4 * RW + 4 * f);
-                            pv[0] = p4.x, pv[1] = p4.y, pv[2] = p4.z, pv[3] = p4.w;
-                            if (cp.xmode) {
-                                const float4 x4 = *(const float4 *)(Raw + 5 * RW + 4 * f);
-                                xv[0] = x4.x, xv[1] = x4.y, xv[2] = x4.z, xv[3] = x4.w;
-                            }
-                        }
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int cw = cw0 + k;
-                            const bool valid = P.pv && cw >= P.lo3 && cw < P.hi3;
-                            const bool own = valid && any_own && cw >= P.olo3 && cw < P.ohi3;
-                            if (!valid) val[k] = 0.0f;
-                            if (own) {
-                                const float ur = dv[k] * rv[k];
-                                const float po = fmaf(beta, pv[k], ur);
-                                cp.snew[gw + k] = so[k];
-                                cp.rnew[gw + k] = rno[k];
-                                cp.p[gw + k] = po;
-                                if (cp.xmode)
-                                    cp.xu[gw + k] =
-                                        cp.xmode == 2 ? fmaf(c1, pv[k], fmaf(alpha, ur, xv[k])) : fmaf(alpha, po, xv[k]);
-                                g_ru = fmaf(rno[k], val[k], g_ru);
-                                g_rr = dv[k] != 0.0f ? fmaf(rno[k], rno[k], g_rr) : g_rr;
-                            }
+                            g_rr = dv[k] != 0.0f ? fmaf(rno[k], rno[k], g_rr) : g_rr;
                         }
                     }
                 }
@@ -547,7 +523,6 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
         }
     };
     float ex[EPT];
-    bool eok[EPT];
     // (y, z) offset ey nz + ez of element tid + q NT within an element plane, -1 outside the
     // grid (loop-invariant: the integer division by NZ runs once per pass)
     int eoff[EPT];
@@ -561,18 +536,12 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
     auto issue_eplane = [&](int j) {
 #pragma unroll
         for (int q = 0; q < EPT; ++q) {
-            eok[q] = j >= 0 && j < nx && eoff[q] >= 0;
-            ex[q] = eok[q] ? x[j * eplane + eoff[q]] : 0.0f;
+            ex[q] = j >= 0 && j < nx && eoff[q] >= 0 ? x[j * eplane + eoff[q]] : 0.0f;
         }
     };
-    // PLAIN: x holds densities and the law gives the moduli; CG modes: x already holds the
-    // moduli E(x_e) of the solve (issue_eplane leaves 0 outside the grid)
+    // x holds the moduli E(x_e) of the solve (issue_eplane leaves 0 outside the grid)
     auto commit_eplane = [&](int slot) {
-        if (CG)
-            Es2[slot * NT + tid] = make_float2(ex[0], ex[1]);
-        else
-            Es2[slot * NT + tid] =
-                make_float2(eok[0] ? modulus(law, ex[0]) : 0.0f, eok[1] ? modulus(law, ex[1]) : 0.0f);
+        Es2[slot * NT + tid] = make_float2(ex[0], ex[1]);
     };
     // Index in Bdf of the z+1-side contribution (cy, c = 0) of element e - 1, for an element e
     // in lane 0; component c adds 2 c.
@@ -642,13 +611,6 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
         if (more_elems) issue_eplane(i + 1);
         const bool out_plane = EDGE || i >= xs;
         const bool shared = EDGE && ((i == xs && xs > 0) || (i == xe && xe < nx));  // added, not stored
-        uint8_t om[EPT];
-#pragma unroll
-        for (int q = 0; q < EPT; ++q) {
-            const int l = tid + q * NT;
-            const bool ok = out_plane && l >= H && F0 - H + l < S;
-            om[q] = (!CG && ok && mask) ? mask[(int64_t)i * S + F0 - H + l] : (uint8_t)0;
-        }
 
         // ---- element plane i: elements tid and tid + NT as the two lanes of a float2 ----
         // h: the contributions of element planes i - 1 (carried) and i to node plane i, summed
@@ -664,7 +626,7 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
 #pragma unroll
                 for (int c = 0; c < 3; ++c) v[b][c] = make_float2(src[c], src[c + 3 * NT]);
             }
-            modal_element2<true>(v, E, km);
+            modal_element2(v, E, km);
 #pragma unroll
             for (int b = 0; b < 4; ++b)
 #pragma unroll
@@ -716,14 +678,12 @@ __device__ __forceinline__ bool modal_pass(const ModalGeom &G, const float *__re
                     const float tl = Bdf[max(bl[q], 0) + 2 * c], tm = Bdf[max(bm[q], 0) + 2 * c];
                     s += bl[q] >= 0 ? tl : 0.0f;
                     s += bm[q] >= 0 ? tm : 0.0f;
-                    // PCG modes leave w unmasked: 1/diag = 0 keeps u, p and x at zero on fixed
-                    // DOFs whatever w holds there, and r.r skips them (the plain apply masks)
-                    yc[c] = (!CG && ((om[q] >> c) & 1)) ? 0.0f : s;
+                    // w stays unmasked: 1/diag = 0 keeps u, p and x at zero on fixed DOFs whatever
+                    // w holds there, and r.r skips them
+                    yc[c] = s;
                 }
-                if (CG) {
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) g_wu = fmaf(Pu[3 * l + c], yc[c], g_wu);
-                }
+                for (int c = 0; c < 3; ++c) g_wu = fmaf(Pu[3 * l + c], yc[c], g_wu);
                 float *yo = y + 3 * ((int64_t)i * S + nflat[q]);
                 if (shared) {
 #pragma unroll
@@ -842,35 +802,29 @@ __device__ __forceinline__ void cg_fold(CgState &s, const PcgScalars *sc, const 
 // phase: k mod 6 for the k-th launch of a solve (the graph loop and the host loops know it
 // statically); par = k & 1. MODE_CG reads state slot par ^ 1 and partial slot par ^ 1, writes
 // state slot par (block 0) and partial slot par; w rotates by k mod 3 (CgArgs).
-template <int NT, int EPT, int MAXV, int MODE>
+template <int NT, int EPT, int MAXV>
 __global__ void __launch_bounds__(NT, 2)
-    apply_modal_kernel(ModalGeom G, const float *__restrict__ x, const float *__restrict__ p, float *__restrict__ y,
-                       const uint8_t *__restrict__ mask, Law<float> law, const ModalK km, CgArgs ca, int phase) {
+    apply_modal_kernel(ModalGeom G, const float *__restrict__ x, const ModalK km, CgArgs ca, int phase) {
     extern __shared__ float4 smem4[];
     __shared__ float2 sred[3 * 32];
     const int tid = threadIdx.x;
     const int nblk = gridDim.x * gridDim.y;
     const int bid = blockIdx.x + gridDim.x * blockIdx.y;
     const int par = phase & 1;
-    CgPass cp{0.0f, 0.0f, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
-    if (MODE == MODE_CG) {
-        // Launch k runs iteration k while the solve lasts, so the vector parity is the launch
-        // parity (and w cycles with k mod 3): the first plane's copies go out before the state
-        // is known. Selects, not dynamic indices (those would copy the parameter arrays to the
-        // stack).
-        const bool odd = par;
-        const int w3 = phase >= 3 ? phase - 3 : phase;
-        float *r_c = odd ? ca.r[1] : ca.r[0], *r_n = odd ? ca.r[0] : ca.r[1];
-        float *s_c = odd ? ca.s[1] : ca.s[0], *s_n = odd ? ca.s[0] : ca.s[1];
-        float *w_c = w3 == 0 ? ca.w[0] : w3 == 1 ? ca.w[1] : ca.w[2];
-        float *w_n = w3 == 0 ? ca.w[1] : w3 == 1 ? ca.w[2] : ca.w[0];
-        float *w_z = w3 == 0 ? ca.w[2] : w3 == 1 ? ca.w[0] : ca.w[1];
-        // x is updated on odd launches only, two iterations at a time
-        cp = CgPass{0.0f, 0.0f, r_c, w_c, s_n, ca.dinv, r_n, s_c, ca.p, ca.xu, w_z, ca.sc, odd ? 2 : 0};
-        y = w_n;
-    }
+    // Launch k runs iteration k while the solve lasts, so the vector parity is the launch
+    // parity (and w cycles with k mod 3): the first plane's copies go out before the state
+    // is known. Selects, not dynamic indices (those would copy the parameter arrays to the
+    // stack).
+    const bool odd = par;
+    const int w3 = phase >= 3 ? phase - 3 : phase;
+    float *r_c = odd ? ca.r[1] : ca.r[0], *r_n = odd ? ca.r[0] : ca.r[1];
+    float *s_c = odd ? ca.s[1] : ca.s[0], *s_n = odd ? ca.s[0] : ca.s[1];
+    float *w_c = w3 == 0 ? ca.w[0] : w3 == 1 ? ca.w[1] : ca.w[2];
+    float *w_n = w3 == 0 ? ca.w[1] : w3 == 1 ? ca.w[2] : ca.w[0];
+    float *w_z = w3 == 0 ? ca.w[2] : w3 == 1 ? ca.w[0] : ca.w[1];
+    // x is updated on odd launches only, two iterations at a time
+    const CgPass cp{0.0f, 0.0f, r_c, w_c, s_n, ca.dinv, r_n, s_c, ca.p, ca.xu, w_z, ca.sc, odd ? 2 : 0};
     auto pre = [&](float &alpha, float &beta, float &alpha_prev) -> bool {
-        if (MODE != MODE_CG) return true;
         const PcgScalars *sc = ca.sc;
         CgState s = sc->st[par ^ 1];
         if (!sc->freeze) {
@@ -897,17 +851,13 @@ __global__ void __launch_bounds__(NT, 2)
         return !s.done;
     };
     float sums[3];
-    if (!modal_pass<NT, EPT, MAXV, MODE>(G, x, p, y, mask, law, km, cp, (float *)smem4, blockIdx.x, blockIdx.y, sums,
-                                         pre))
-        return;
-    if (MODE == MODE_CG) {
-        df32 bs[3] = {{sums[0], 0.0f}, {sums[1], 0.0f}, {sums[2], 0.0f}};
-        block_sum_df<3>(bs, sred);
-        if (tid == 0) {
-            float2 *part = (float2 *)ca.partials + par * 3 * nblk;
+    if (!modal_pass<NT, EPT, MAXV, MODE_CG>(G, x, w_n, km, cp, (float *)smem4, blockIdx.x, blockIdx.y, sums, pre)) return;
+    df32 bs[3] = {{sums[0], 0.0f}, {sums[1], 0.0f}, {sums[2], 0.0f}};
+    block_sum_df<3>(bs, sred);
+    if (tid == 0) {
+        float2 *part = (float2 *)ca.partials + par * 3 * nblk;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) part[k * nblk + bid] = make_float2(bs[k].hi, bs[k].lo);
-        }
+        for (int k = 0; k < 3; ++k) part[k * nblk + bid] = make_float2(bs[k].hi, bs[k].lo);
     }
 }
 
@@ -970,54 +920,50 @@ inline int modal_resident(const gbsimp_ctx *ctx, const void *kern, int &reg_cach
 
 // Sets the kernel's dynamic shared-memory limit once per device (host calls only; done before
 // any graph capture) and returns resident CTAs per SM for this z extent, or < 0 on error.
-template <int MODE, int MAXV>
+template <int MAXV>
 inline int modal_prepare_one(const gbsimp_ctx *ctx, int nz) {
-    auto kern = apply_modal_kernel<kModalNT, kModalEPT, MAXV, MODE>;
-    constexpr bool cg = MODE != MODE_PLAIN;
+    auto kern = apply_modal_kernel<kModalNT, kModalEPT, MAXV>;
     static int set_cache[128] = {};  // benign races: every thread stores the same values
     static int reg_cache[128] = {};
     const int dev = ctx->device >= 0 && ctx->device < 128 ? ctx->device : 0;
     if (!set_cache[dev]) {
-        const int smax = (int)modal_smem_bytes<kModalNT, kModalEPT>(446, cg);
+        const int smax = (int)modal_smem_bytes<kModalNT, kModalEPT>(446);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
         if (e != cudaSuccess) return -cuda_error(e, "cudaFuncSetAttribute(apply_modal_kernel)");
         set_cache[dev] = 1;
     }
-    return modal_resident(ctx, (const void *)kern, reg_cache[dev], modal_smem_bytes<kModalNT, kModalEPT>(nz, cg));
+    return modal_resident(ctx, (const void *)kern, reg_cache[dev], modal_smem_bytes<kModalNT, kModalEPT>(nz));
 }
 
-template <int MODE>
 inline int modal_prepare(const gbsimp_ctx *ctx, int nz) {
-    return modal_short(nz) ? modal_prepare_one<MODE, 2>(ctx, nz) : modal_prepare_one<MODE, 3>(ctx, nz);
+    return modal_short(nz) ? modal_prepare_one<2>(ctx, nz) : modal_prepare_one<3>(ctx, nz);
 }
 
-// CTAs of the modal kernel's launch for a grid (the partial sums of one MODE_CG pass).
-template <int MODE>
+// CTAs of the modal kernel's launch for a grid (the partial sums of one pass).
 inline int modal_blocks(const gbsimp_ctx *ctx, int nx, int ny, int nz) {
-    const int per_sm = modal_prepare<MODE>(ctx, nz);
+    const int per_sm = modal_prepare(ctx, nz);
     if (per_sm < 0) return per_sm;
-    const dim3 g = modal_grid(modal_geom(nx, ny, nz, ctx->num_sms, per_sm, MODE == MODE_CG));
+    const dim3 g = modal_grid(modal_geom(nx, ny, nz, ctx->num_sms, per_sm, true));
     return (int)(g.x * g.y);
 }
 
-// Launches the modal kernel (MODE_PLAIN: y = D K D p; MODE_CG: one PCG iteration, phase =
-// launch index mod 6).
-template <int MODE>
-inline int launch_modal(const gbsimp_ctx *ctx, int nx, int ny, int nz, const Law<float> &law, const float *x,
-                        const float *p, float *y, const uint8_t *mask, const CgArgs &ca, cudaStream_t st,
-                        int phase = 0) {
-    const int per_sm = modal_prepare<MODE>(ctx, nz);
+// Launches the modal kernel: one PCG iteration, phase = launch index mod 6.
+inline int launch_modal(const gbsimp_ctx *ctx, int nx, int ny, int nz, const float *x, const CgArgs &ca,
+                        cudaStream_t st, int phase) {
+    const int per_sm = modal_prepare(ctx, nz);
     if (per_sm < 0) return -per_sm;
-    const size_t smem = modal_smem_bytes<kModalNT, kModalEPT>(nz, MODE != MODE_PLAIN);
-    const ModalGeom g = modal_geom(nx, ny, nz, ctx->num_sms, per_sm, MODE == MODE_CG);
+    const size_t smem = modal_smem_bytes<kModalNT, kModalEPT>(nz);
+    const ModalGeom g = modal_geom(nx, ny, nz, ctx->num_sms, per_sm, true);
     if (modal_short(nz))
-        apply_modal_kernel<kModalNT, kModalEPT, 2, MODE>
-            <<<modal_grid(g), kModalNT, smem, st>>>(g, x, p, y, mask, law, ctx->km, ca, phase);
+        apply_modal_kernel<kModalNT, kModalEPT, 2><<<modal_grid(g), kModalNT, smem, st>>>(g, x, ctx->km, ca, phase);
     else
-        apply_modal_kernel<kModalNT, kModalEPT, 3, MODE>
-            <<<modal_grid(g), kModalNT, smem, st>>>(g, x, p, y, mask, law, ctx->km, ca, phase);
+        apply_modal_kernel<kModalNT, kModalEPT, 3><<<modal_grid(g), kModalNT, smem, st>>>(g, x, ctx->km, ca, phase);
     GBS_LAUNCH_CHECK("apply_modal_kernel");
     return GBS_OK;
 }
+
+// y = D K(x) D p in one launch (apply_plain.cu; modal_fits(nz)).
+int apply_plain(const gbsimp_ctx *ctx, int nx, int ny, int nz, const Law<float> &law, const float *x, const float *p,
+                float *y, const uint8_t *mask, cudaStream_t st);
 
 }  // namespace gbs

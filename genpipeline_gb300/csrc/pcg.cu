@@ -82,7 +82,7 @@ static size_t pcg_partials(int nx, int ny, int nz) {
 // The one-kernel PCG's launch on this grid writes 6 partial sums per CTA: refuse a workspace
 // that cannot hold them (a wave larger than kModalMaxWave CTAs).
 static int check_modal_partials(const gbsimp_ctx *ctx, int nx, int ny, int nz, const PcgWs &w) {
-    const int nblk = modal_blocks<MODE_CG>(ctx, nx, ny, nz);
+    const int nblk = modal_blocks(ctx, nx, ny, nz);
     if (nblk < 0) return -nblk;
     if (6 * (size_t)nblk > w.partial_count)
         return set_error(GBS_EINVAL, "PCG: the launch needs more partial sums than the workspace holds");
@@ -467,7 +467,7 @@ static int pcg_iteration(const gbsimp_ctx *ctx, int nx, int ny, int nz, const La
                          const uint8_t *mask, float *u, const PcgWs &w, cudaStream_t st, cudaEvent_t after_k1,
                          int phase) {
     if (use_modal(ctx, nz)) {  // reads the moduli w.E of the setup, not x
-        int rc = launch_modal<MODE_CG>(ctx, nx, ny, nz, law, w.E, nullptr, nullptr, mask, cg_args(w, u), st, phase);
+        int rc = launch_modal(ctx, nx, ny, nz, w.E, cg_args(w, u), st, phase);
         if (rc) return rc;
         if (after_k1) GBS_CUDA_TRY(cudaEventRecord(after_k1, st));
         return GBS_OK;
@@ -619,8 +619,8 @@ __global__ void __launch_bounds__(NT, 2)
         const int c = it & 1, nc = c ^ 1;
         const CgPass cp{alpha.hi, beta.hi, ca.r[c], ca.w[c], ca.s[nc], ca.dinv, ca.r[nc], ca.s[c], ca.p, ca.xu, nullptr, ca.sc, 1};
         float sums[3];
-        modal_pass<NT, EPT, MAXV, MODE_CG_FUSED>(G, D.x, nullptr, ca.w[nc], D.mask, law, km, cp, (float *)smem4, tile, seg,
-                                                 sums, [](float &, float &, float &) { return true; });
+        modal_pass<NT, EPT, MAXV, MODE_CG_FUSED>(G, D.x, ca.w[nc], km, cp, (float *)smem4, tile, seg, sums,
+                                                 [](float &, float &, float &) { return true; });
         __threadfence();
         target += nblk;
         df32 tot[3];
@@ -691,9 +691,9 @@ static int fused_plan(const gbsimp_ctx *ctx, const FusedItem *items, int n, Fuse
     static int reg_cache[2][128] = {};
     const int dev = ctx->device >= 0 && ctx->device < 128 ? ctx->device : 0;
     int &ready = ready_cache[small ? 0 : 1][dev];
-    const size_t smem = modal_smem_bytes<kModalNT, kModalEPT>(max_nz, true);
+    const size_t smem = modal_smem_bytes<kModalNT, kModalEPT>(max_nz);
     if (ready == 0) {
-        const int smax = (int)modal_smem_bytes<kModalNT, kModalEPT>(446, true);
+        const int smax = (int)modal_smem_bytes<kModalNT, kModalEPT>(446);
         int coop = 0;
         const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) == cudaSuccess &&
                         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop;
@@ -849,7 +849,7 @@ static int pcg_iteration(const gbsimp_ctx *ctx, int nx, int ny, int nz, const La
 // Publishes the state after one-kernel PCG launches (last launch of parity `last`).
 static int cg_publish(const gbsimp_ctx *ctx, int nx, int ny, int nz, const PcgWs &w, int last, cudaStream_t st) {
     if (!use_modal(ctx, nz)) return GBS_OK;
-    const int nblk = modal_blocks<MODE_CG>(ctx, nx, ny, nz);
+    const int nblk = modal_blocks(ctx, nx, ny, nz);
     if (nblk < 0) return -nblk;
     cg_fold_kernel<<<1, 256, 0, st>>>(nblk, last, w.partials, w.sc);
     GBS_LAUNCH_CHECK("cg_fold_kernel");
@@ -896,7 +896,7 @@ static int launch_loop_graph(const gbsimp_ctx *ctx, int nx, int ny, int nz, cons
         gc->map.clear();
     }
     if (modal) {
-        const int r = modal_prepare<MODE_CG>(ctx, nz);
+        const int r = modal_prepare(ctx, nz);
         if (r < 0) return -r;
     }
     if (!gc->cap) GBS_CUDA_TRY(cudaStreamCreateWithFlags(&gc->cap, cudaStreamNonBlocking));
@@ -1720,7 +1720,7 @@ int solve_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *l
             }
         }
         if (finish_left) {
-            const int nblk = modal_blocks<MODE_CG>(ctx, nx, ny, nz);
+            const int nblk = modal_blocks(ctx, nx, ny, nz);
             if (nblk < 0) return -nblk;
             // every block folds the ~300 partial sums itself: vec_blocks' cap (8 blocks per SM)
             // keeps those redundant reads small
@@ -1982,7 +1982,7 @@ extern "C" int gbsimp_time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, co
         return GBS_OK;
     }
     if (modal) {
-        const int r = modal_prepare<MODE_CG>(ctx, nz);
+        const int r = modal_prepare(ctx, nz);
         if (r < 0) return -r;
     }
     GraphCache *gc = (GraphCache *)ctx->graphs;
@@ -1994,8 +1994,7 @@ extern "C" int gbsimp_time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, co
     PcgArgs pa{w.r, w.dinv, w.p0, w.p1, xu, w.partials, w.sc};
     for (int i = 0; i < reps && rc == GBS_OK; ++i) {
         if (modal) {
-            rc = launch_modal<MODE_CG>(ctx, nx, ny, nz, law, w.E, nullptr, nullptr, node_mask, cg_args(w, xu), gc->cap,
-                                       i % 6);
+            rc = launch_modal(ctx, nx, ny, nz, w.E, cg_args(w, xu), gc->cap, i % 6);
         } else {
             TileArgs<float> A{nx, ny, nz, x, nullptr, w.ap, node_mask};
             const dim3 g = tile_grid<TileF>(nx, ny, nz), b = tile_block<TileF>();
