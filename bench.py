@@ -204,7 +204,7 @@ def _measured_peak():
 def _profiled_traffic(workload="simp64"):
     """DRAM bytes per launch of the one-kernel PCG iteration from the committed ncu summary of the
     workload."""
-    name = {"simp64": "cg_iteration__simp_64cube.md", "c4": "cg_iteration__simp_192x96x96.md"}.get(workload)
+    name = {"simp64": "pcg_chip__64cube.md", "c4": "cg_iteration__simp_192x96x96.md"}.get(workload)
     if name is None:
         return None
     path = os.path.join(ROOT, "profiles", name)
@@ -382,7 +382,7 @@ def measure_rows(xphys64=None):
 
 
 def run_apply(a):
-    """The bare stiffness apply y = D K(x) D p (`apply_modal_kernel<PLAIN>`, no masks) at 64^3
+    """The bare stiffness apply y = D K(x) D p (`apply_plain_kernel`, no masks) at 64^3
     and 192x96x96 on seeded densities U(0.1, 1) and a seeded N(0, 1) vector. Warm: 20
     back-to-back launches, median of 5 groups. Cold: single launches after a 256 MB L2 flush,
     median of `--steps` (at least 5). Algorithmic bytes are 4*(2 n_dof + n_elem): p in, y out,
@@ -446,7 +446,7 @@ def run_apply(a):
             "vs_baseline": None, "dtype": "f32", "data": "synthetic", "impl": "ours",
             "config": {"workload": "stiffness_apply", "grids": list(grids), "densities": "U(0.1, 1), seed 0",
                        "law": COMMON["law"], "l2": "flushed (256 MB write) before each cold launch"},
-            "roofline": {"bound": "hbm", "kernel": "apply_modal_kernel<PLAIN>", "achieved": c4["cold_GBs"],
+            "roofline": {"bound": "hbm", "kernel": "apply_plain_kernel", "achieved": c4["cold_GBs"],
                          "peak": peak, "peak_source": peak_src, "unit": "GB/s", "frac": c4["cold_frac"],
                          "traffic": None},
             "grids": grids, "gpu_launches": int(launches), "clocks": clk}
@@ -501,7 +501,7 @@ def measure_c4(peak: float):
     """192x96x96 (1,769,472 elements, 5,447,811 DOFs) on seeded densities U(0.1, 1) with the
     line-load case's Dirichlet mask: the one-kernel PCG iteration (gbsimp_time_pcg_apply: 50
     graph-replayed launches, CUDA events on the stream, frozen scalars) and the bare stiffness
-    apply y = D K(x) D p (apply_modal_kernel<PLAIN>), warm (20 back-to-back launches, median of
+    apply y = D K(x) D p (apply_plain_kernel), warm (20 back-to-back launches, median of
     5) and cold (one launch after a 256 MB L2 flush, median of 5). The PCG vectors (about
     218 MB) do not fit in the 129 MB L2."""
     import torch
@@ -544,10 +544,10 @@ def measure_c4(peak: float):
     cold = statistics.median(cold)
     apply_bytes = 4 * (2 * nd + ne)
     return {"workload": "192x96x96, densities U(0.1,1) seed 0, x=0 clamped (line-load case's mask)",
-            "pcg_iteration": {"kernel": "apply_modal_kernel<CG>", "launch_us": per_launch * 1e6,
+            "pcg_iteration": {"kernel": "apply_modal_kernel", "launch_us": per_launch * 1e6,
                               "alg_bytes_per_launch": pcg_bytes, "achieved_GBs": pcg_bytes / per_launch / 1e9,
                               "frac": pcg_bytes / per_launch / 1e9 / peak, "traffic": _profiled_traffic("c4")},
-            "bare_apply": {"kernel": "apply_modal_kernel<PLAIN>", "warm_us": warm * 1e6, "cold_us": cold * 1e6,
+            "bare_apply": {"kernel": "apply_plain_kernel", "warm_us": warm * 1e6, "cold_us": cold * 1e6,
                            "alg_bytes_per_launch": apply_bytes, "cold_GBs": apply_bytes / cold / 1e9,
                            "cold_frac": apply_bytes / cold / 1e9 / peak, "warm_frac": apply_bytes / warm / 1e9 / peak},
             "peak_GBs": peak}
@@ -782,7 +782,9 @@ def run_ours(a):
         # out; x read and written every other iteration (two-step update): 10 words per DOF
         # on average, the basis of one standard Jacobi-PCG iteration
         alg_bytes = 4 * (10 * nd + ne)
-        kname = "apply_modal_kernel<CG> (one single-reduction PCG iteration: s, r, u staging, w = DKDu, p, x)"
+        # (a grid that the chip holds moves none of them: frac then says how much faster than a pass
+        # over memory the iteration is)
+        kname = "one single-reduction PCG iteration: s, r, u, w = DKDu, p, x (pcg_chip_kernel, or apply_modal_kernel)"
     else:
         alg_bytes = 4 * (7 * nd + ne)  # r, dinv, p_old, x_u, x in; p_new, Ap, x_u out
         kname = "apply_tile_kernel<PCG> (K(x)p fused with p = z + beta p, x update, p.Ap)"
