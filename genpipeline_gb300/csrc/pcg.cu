@@ -1,9 +1,11 @@
 // pcg.cu -- Jacobi-PCG drivers: FP32 matrix-free PCG, FP32-inner / FP64-outer defect
 // correction, and a CSR PCG for the pcg_solve_cuda contract.
 //
-// Two forms of the same Jacobi-PCG (simp_solver_gpu.py:328-379: z = r/diag, stop when
+// Three forms of the same Jacobi-PCG (simp_solver_gpu.py:328-379: z = r/diag, stop when
 // ||r|| < rtol ||D b||):
-// - modal element (isotropic cube Ke): one launch per iteration, the single-reduction form
+// - modal element (isotropic cube Ke), a grid that the chip holds: all iterations in one launch
+//   (pcg_chip.cu).
+// - modal element, a larger grid: one launch per iteration, the single-reduction form
 //   (apply_modal.cuh, MODE_CG): the staging of the apply operand u_{i+1} = M r_{i+1} also
 //   forms s_i and r_{i+1}, the owned nodes update p (and x on odd launches, two iterations
 //   at once), and each block writes its sums of r.u, w.u and r.r; the next launch folds them
