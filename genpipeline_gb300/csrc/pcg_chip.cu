@@ -763,8 +763,9 @@ __global__ void __launch_bounds__(kChipNT, 1)
         return;
     }
     // ---- the iterate out; a paused solve's state too -------------------------------------------
-    // x owes the last iteration's step when that one did not update it
+    // x owes the last iteration's step when that one did not update it; x = 0 when D b = 0, whatever x0
     const float owed = kTight || two ? alpha_prev : 0.0f;
+    const bool zero = !fresh && S.bnorm == 0.0;
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int n = tid + kChipNT * q;
@@ -779,7 +780,7 @@ __global__ void __launch_bounds__(kChipNT, 1)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float2 w = add2(W0[3 * n + c], W1[3 * n + c]), x = Xs[3 * n + c];
-                I.u[g0 + c] = fmaf(owed, h ? p[q][c].y : p[q][c].x, h ? x.y : x.x);
+                I.u[g0 + c] = zero ? 0.0f : fmaf(owed, h ? p[q][c].y : p[q][c].x, h ? x.y : x.x);
                 if (!done) {
                     I.r[g0 + c] = h ? r[q][c].y : r[q][c].x;
                     I.w[g0 + c] = h ? w.y : w.x;
