@@ -234,6 +234,13 @@ extern "C" int gbsimp_set_ke(gbsimp_ctx *ctx, const double *ke576) {
     return GBS_OK;
 }
 
+extern "C" int gbsimp_set_diagnostic(gbsimp_ctx *ctx, int key, int64_t value) {
+    if (!ctx || key < 1 || key >= (int)(sizeof ctx->diag / sizeof *ctx->diag) || value > INT32_MAX - 1)
+        return set_error(GBS_EINVAL, "gbsimp_set_diagnostic: bad arguments");
+    ctx->diag[key] = value < 0 ? 0 : value + 1;
+    return GBS_OK;
+}
+
 extern "C" int gbsimp_get_ke(const gbsimp_ctx *ctx, double *ke576) {
     if (!ctx || !ke576) return set_error(GBS_EINVAL, "gbsimp_get_ke: bad arguments");
     memcpy(ke576, ctx->ke, sizeof ctx->ke);

@@ -434,9 +434,13 @@ struct gbsimp_ctx {
     gbs::ModalKD kmd;       // the same in FP64
     unsigned ke_version;    // bumped by every set_ke (keys the graph cache)
     void *graphs;           // gbs::GraphCache* (pcg.cu): instantiated device-loop graphs
+    int64_t diag[2];        // gbsimp_set_diagnostic, by key: the value + 1, 0 where the default holds
 };
 
 namespace gbs {
+// Polls after which a wait for another block's packet runs out: a poll is an L2 round trip, so that is
+// two seconds or so (gbsimp_set_diagnostic: after one look).
+inline unsigned wait_polls(const gbsimp_ctx *ctx) { return ctx->diag[GBSIMP_DIAG_TIMEOUT] == 1 ? 0u : 1u << 22; }
 int set_error(int code, const char *fmt, ...);
 int cuda_error(cudaError_t e, const char *what);
 void count_launches(int n);

@@ -1134,7 +1134,7 @@ int oc_run_impl(const gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin, cons
     if (cb > 0) {
         const int64_t per = (n + (int64_t)nb * kCoopThreads - 1) / ((int64_t)nb * kCoopThreads);
         int keep = (int)std::min<int64_t>(per, kCoopKeep) * kCoopThreads;
-        unsigned polls = 1u << 22;  // per wait; a poll is an L2 round trip, so two seconds or so
+        unsigned polls = wait_polls(ctx);
         void *args[] = {(void *)&n, (void *)&P, (void *)&x, (void *)&dc, (void *)&preserved, (void *)&w.w,
                         (void *)&box, (void *)&w.sc, (void *)&xnew, (void *)&keep, (void *)&polls};
         GBS_CUDA_TRY(cudaLaunchCooperativeKernel((void *)oc_coop_kernel, dim3((unsigned)nb), dim3(kCoopThreads), args,
@@ -1196,7 +1196,7 @@ extern "C" int gbsimp_oc_result(gbsimp_ctx *ctx, const void *ws, double *lambda_
     if (lambda_out) *lambda_out = h.lfinal;
     if (steps_out) *steps_out = h.steps;
     if (h.status == GBS_ETIMEOUT)
-        return set_error(GBS_ETIMEOUT, "gbsimp_oc_result: a grid barrier wait of the OC update ran out");
+        return set_error(GBS_ETIMEOUT, "gbsimp_oc_result: a wait of the OC update on another block ran out");
     return GBS_OK;
 }
 

@@ -1462,9 +1462,10 @@ __global__ void scale_dd_kernel(int64_t nd, const float2 *__restrict__ r, const 
 }
 
 // u += ||r|| d (one FP64 fma), fixed DOFs zero, and its double-float split for the next
-// residual (integer conversions: f2d, dd_split).
-__global__ void correct_dd_kernel(int64_t nd, const float *__restrict__ d, const OuterScalars *os,
+// residual (integer conversions: f2d, dd_split). A solve whose wait ran out has no d: u stays.
+__global__ void correct_dd_kernel(int64_t nd, const float *__restrict__ d, const OuterScalars *os, const PcgScalars *sc,
                                   const uint8_t *__restrict__ mask, double *u, float2 *udd) {
+    if (sc->status == GBS_ETIMEOUT) return;
     const double s = os->rnorm;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nd; i += (int64_t)gridDim.x * blockDim.x) {
         const bool fx = dof_fixed(mask, i);
@@ -1543,8 +1544,9 @@ __global__ void scale_to_f32_kernel(int64_t nd, const double *__restrict__ r, co
     }
 }
 
-__global__ void correct64_kernel(int64_t nd, const float *__restrict__ d, const OuterScalars *os,
+__global__ void correct64_kernel(int64_t nd, const float *__restrict__ d, const OuterScalars *os, const PcgScalars *sc,
                                  const uint8_t *__restrict__ mask, double *u) {
+    if (sc->status == GBS_ETIMEOUT) return;
     const double s = os->rnorm;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nd; i += (int64_t)gridDim.x * blockDim.x)
         u[i] = dof_fixed(mask, i) ? 0.0 : fma((double)d[i], s, u[i]);
@@ -1576,13 +1578,13 @@ static int outer_residual(const gbsimp_ctx *ctx, int nx, int ny, int nz, const g
 }
 
 // u += d / scale, and with the double-float residual the split of the new u.
-static int outer_correct(const gbsimp_ctx *ctx, int64_t nd, const uint8_t *mask, double *u, bool dd,
+static int outer_correct(const gbsimp_ctx *ctx, int64_t nd, const PcgScalars *sc, const uint8_t *mask, double *u, bool dd,
                          const SolveWs &w, cudaStream_t st) {
     if (dd) {
-        correct_dd_kernel<<<ew_blocks(ctx, nd), 256, 0, st>>>(nd, w.d32, w.os, mask, u, w.udd);
+        correct_dd_kernel<<<ew_blocks(ctx, nd), 256, 0, st>>>(nd, w.d32, w.os, sc, mask, u, w.udd);
         GBS_LAUNCH_CHECK("correct_dd_kernel");
     } else {
-        correct64_kernel<<<ew_blocks(ctx, nd), 256, 0, st>>>(nd, w.d32, w.os, mask, u);
+        correct64_kernel<<<ew_blocks(ctx, nd), 256, 0, st>>>(nd, w.d32, w.os, sc, mask, u);
         GBS_LAUNCH_CHECK("correct64_kernel");
     }
     return GBS_OK;
@@ -1668,8 +1670,8 @@ int solve_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *l
             pending = nullptr;
             total += ps.iter;
             count_launches(ps.trips * launches_per_trip(ctx, nz));  // graph loop trips (0 for the persistent kernel)
-            // a failed inner solve ends the loop; its correction (zero when it made no step)
-            // is in u and the residual above is the one of the corrected u
+            // a failed inner solve ends the loop; its correction (zero when it made no step, none after
+            // a timeout) is in u and the residual above is the one of the corrected u
             if (ps.status == GBS_EBREAKDOWN || ps.status == GBS_ENONFINITE || ps.status == GBS_ETIMEOUT)
                 status = ps.status;
         }
@@ -1730,7 +1732,7 @@ int solve_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *l
                                                                      w.os, mask, u, w.udd);
             GBS_LAUNCH_CHECK("cg_finish_dd_kernel");
         } else {
-            rc = outer_correct(ctx, nd, mask, u, dd, w, st);
+            rc = outer_correct(ctx, nd, pw.sc, mask, u, dd, w, st);
             if (rc) return rc;
         }
         if (status != GBS_OK) break;
@@ -2448,7 +2450,8 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
                 }
             }
             SolveWs w = solve_ws(it.ws, it.nx, it.ny, it.nz);
-            int rc = outer_correct(ctx, n_dof_of(it.nx, it.ny, it.nz), it.node_mask, it.u, dd, w, st);
+            int rc = outer_correct(ctx, n_dof_of(it.nx, it.ny, it.nz), pcg_ws(w.pcg, it.nx, it.ny, it.nz).sc, it.node_mask,
+                                   it.u, dd, w, st);
             if (rc) return rc;
             if (it.stats.status != GBS_OK) it.state = 2;
         }

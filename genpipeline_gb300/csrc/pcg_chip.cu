@@ -61,7 +61,7 @@ struct ChipDesign {
     ChipItem it;
 };
 struct ChipTable {
-    int n, pad;
+    int n, late;  // late: the block that reports a timeout at its end (diagnostics), 0: none
     ChipDesign d[kChipMaxDesigns];
 };
 static_assert(sizeof(ChipTable) + 128 <= 4096, "kernel parameters");
@@ -135,6 +135,10 @@ static size_t chip_smem(int slots, int esteps, const ChipShared &n) {
 // each CTA), the scalars' packets (two parities x copies, a 128-byte line each), then the node
 // packets (two parities x CTAs x the largest box).
 __host__ __device__ inline size_t chip_mail(int nblk) { return (((size_t)64 * nblk + 255) & ~(size_t)255) + 2 * kChipCopies * 128; }
+// The launch's flag of a wait that ran out: a word of the first scalars' line that no packet uses.
+__device__ __forceinline__ unsigned *chip_late(float4 *xch, int nblk) {
+    return (unsigned *)((char *)xch + chip_mail(nblk) - 2 * kChipCopies * 128 + 64);
+}
 static size_t chip_xch(int nblk, int stride) {
     return nblk > 1 ? chip_mail(nblk) + 2 * (size_t)nblk * stride * sizeof(float4) : 0;
 }
@@ -753,10 +757,18 @@ __global__ void __launch_bounds__(kChipNT, 1)
         if (!first) ++it;
         first = false;
     }
-    if (status == GBS_ETIMEOUT) {
+    // Whichever block's wait ran out, the solve's status is GBS_ETIMEOUT: the block raises the launch's
+    // flag before it writes the status, the first block looks at the flag after it has written its own, so
+    // that one of the two writes GBS_ETIMEOUT last. Its part of x stays as it came (nobody reads that of
+    // a fresh solve).
+    if (status == GBS_ETIMEOUT || (T.late > 0 && T.late == bid)) {
         if (tid == 0) {
-            sc->iter = it;
-            sc->trips = 0;
+            if (bid == 0) {
+                sc->iter = it;
+                sc->trips = 0;
+            }
+            atomicExch(chip_late(I.xch, nblk), 1u);
+            __threadfence();
             atomicExch(&sc->status, (int)GBS_ETIMEOUT);
             atomicExch(&sc->done, 1);
         }
@@ -804,6 +816,11 @@ __global__ void __launch_bounds__(kChipNT, 1)
         sc->beta = df_value(S.beta);
         sc->trips = 0;
         sc->freeze = S.freeze;
+        __threadfence();
+        if (nblk > 1 && atomicAdd(chip_late(I.xch, nblk), 0u)) {
+            atomicExch(&sc->status, (int)GBS_ETIMEOUT);
+            atomicExch(&sc->done, 1);
+        }
     }
 }
 
@@ -968,6 +985,7 @@ int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cu
     ChipTable T;
     memset(&T, 0, sizeof T);
     T.n = n;
+    T.late = ctx->diag[GBSIMP_DIAG_TIMEOUT] > 1 ? (int)(ctx->diag[GBSIMP_DIAG_TIMEOUT] - 1) : 0;
     int block0 = 0, q = 0;
     size_t smem = 0;
     for (int i = 0; i < n; ++i) {
@@ -989,8 +1007,8 @@ int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cu
         if (T.d[i].nblk > 1)
             GBS_CUDA_TRY(cudaMemsetAsync(items[i].xch, 0, chip_xch(T.d[i].nblk, T.d[i].g.stride), st));
     }
-    unsigned polls = 1u << 22;  // per wait; a poll is an L2 round trip, so two seconds or so
     ModalK km = ctx->km;
+    unsigned polls = wait_polls(ctx);
     void *args[] = {&km, &polls, &budget, &T};
     const cudaError_t e =
         cudaLaunchCooperativeKernel((const void *)chip_kern[v], dim3((unsigned)block0), dim3(kChipNT), args, smem, st);

@@ -220,7 +220,9 @@ int gbsimp_oc_result(gbsimp_ctx *ctx, const void *ws, double *lambda_out, int *s
  * the device: a CUDA graph (cached per buffer set) whose WHILE node repeats 12 iterations
  * while the device-side stop flag is clear, with a hard cap derived from max_iter
  * (GBS_ETIMEOUT). With opts->profile the host launches the iterations instead, checking
- * every opts->check_every iterations, and times each apply launch. Synchronises the stream. */
+ * every opts->check_every iterations, and times each apply launch. On a grid that the chip holds all
+ * iterations run in one cooperative launch; when one of its bounded waits runs out (GBS_ETIMEOUT), u is
+ * unspecified here, and stays as the last outer round left it in gbsimp_solve. Synchronises the stream. */
 size_t gbsimp_pcg_ws_bytes(int nx, int ny, int nz);
 int gbsimp_pcg_f32(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *law,
                    const float *x, const float *b, const uint8_t *node_mask, float *u,
@@ -365,6 +367,13 @@ int gbsimp_pcg_csr_f32(gbsimp_ctx *ctx, int64_t n, const int32_t *row_ptr,
 size_t gbsimp_barrier_selftest_ws_bytes(void);
 int gbsimp_barrier_selftest(gbsimp_ctx *ctx, int extra_arrivals, double wait_seconds, int *status_out,
                             void *ws, size_t ws_bytes, void *stream);
+
+/* Diagnostics of one context, for tests (no counterpart in the reference). A negative value, the
+ * default, switches a key off. Not to be set while a call on the context is running.
+ * GBSIMP_DIAG_TIMEOUT: 0: the waits of the on-chip PCG and of the OC update for other blocks run out
+ * after one look; b > 0: block b of an on-chip PCG reports a wait that ran out at its end. */
+enum { GBSIMP_DIAG_TIMEOUT = 1 };
+int gbsimp_set_diagnostic(gbsimp_ctx *ctx, int key, int64_t value);
 
 /* ---- reductions used by the host loops -------------------------------------------- */
 /* out (device double) = sum_i a_i * b_i over n FP64 entries, fixed block order. */
