@@ -80,6 +80,7 @@ class SimpOpts(C.Structure):
 
 
 DIAG_TIMEOUT = 1
+DIAG_CHIP = 2
 
 _P = C.c_void_p
 _I = C.c_int

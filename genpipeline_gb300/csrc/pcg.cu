@@ -1107,6 +1107,18 @@ struct ApplyProfile {
     int launches = 0;
 };
 
+struct EventPair {
+    cudaEvent_t e[2] = {};
+    cudaError_t create() {
+        cudaError_t r = cudaEventCreate(&e[0]);
+        return r == cudaSuccess ? cudaEventCreate(&e[1]) : r;
+    }
+    ~EventPair() {
+        for (cudaEvent_t v : e)
+            if (v) cudaEventDestroy(v);
+    }
+};
+
 // ---- the on-chip form (pcg_chip.cu) ---------------------------------------------------------
 // Whenever the grid fits the chip: it is the faster form at every size that does. us per iteration of
 // a solve, streaming in the graph loop -> on the chip: 8x4x4 7.5 -> 1.7, 32x8x8 7.9 -> 3.9, 32^3
@@ -1143,52 +1155,51 @@ static ChipItem chip_item(int nx, int ny, int nz, const PcgWs &w, float *u, void
 // FP32 PCG. u: x0 in, solution out. Returns GBS_OK and fills *out (status inside).
 // With out == nullptr (and no profiling) the solve is only enqueued: the device-driven paths
 // need no host decision, and the caller reads the scalars later (w.sc of the workspace),
-// together with its own.
+// adding the graph loop's launches (trips x launches_per_trip) itself.
+// chip: the on-chip form where the grid fits; returns kChipRefused when its launch is refused, u
+// unchanged (the caller comes again without it).
 int pcg_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *glaw, const float *x, const float *b,
             const uint8_t *mask, float *u, double rtol, int max_iter, int check_every, void *ws, PcgScalars *out,
-            cudaStream_t st, ApplyProfile *prof = nullptr, int fused = 0, unsigned setup_flags = 0,
+            cudaStream_t st, bool chip, ApplyProfile *prof = nullptr, int fused = 0, unsigned setup_flags = 0,
             const float2 *bdd = nullptr, const double *bscale = nullptr, bool *finish_left = nullptr,
             void *scratch = nullptr, size_t scratch_bytes = 0) {
     const int64_t nd = n_dof_of(nx, ny, nz);
     PcgWs w = pcg_ws(ws, nx, ny, nz);
     const Law<float> law = make_law<float>(*glaw);
-    {
-        ChipItem ci = chip_item(nx, ny, nz, w, u, scratch, scratch_bytes);
-        if (chip_ok(ctx, ci)) {
-            ci.fresh = (setup_flags & SETUP_X0_ZERO) && max_iter > 0;
-            ci.b = b;
-            ci.bdd = bdd;
-            ci.bscale = bscale;
-            ci.tol = rtol;
-            ci.max_iter = max_iter;
-            int rc = GBS_OK;
-            if (!ci.fresh)
-                rc = pcg_setup(ctx, nx, ny, nz, glaw, x, b, mask, u, rtol, max_iter, w, st, setup_flags);
-            else if (!(setup_flags & SETUP_KEEP_DINV))
-                rc = setup_diag(ctx, nx, ny, nz, law, x, mask, w, st);
-            if (rc) return rc;
-            cudaEvent_t ev[2] = {};
-            if (prof) {
-                for (auto &e : ev) GBS_CUDA_TRY(cudaEventCreate(&e));
-                GBS_CUDA_TRY(cudaEventRecord(ev[0], st));
-            }
-            rc = chip_run(ctx, &ci, 1, 0, st);
-            if (rc) return rc;
-            if (prof) GBS_CUDA_TRY(cudaEventRecord(ev[1], st));
-            if (!out && !prof) return GBS_OK;
-            PcgScalars h;
-            rc = read_scalars(w.sc, &h, st);
-            if (rc) return rc;
-            if (prof) {
-                float ms = 0.0f;
-                GBS_CUDA_TRY(cudaEventElapsedTime(&ms, ev[0], ev[1]));
-                prof->seconds += 1e-3 * ms;
-                prof->launches += h.iter;
-                for (auto &e : ev) cudaEventDestroy(e);
-            }
-            if (out) *out = h;
-            return GBS_OK;
+    ChipItem ci = chip_item(nx, ny, nz, w, u, scratch, scratch_bytes);
+    if (chip && chip_ok(ctx, ci)) {
+        ci.fresh = (setup_flags & SETUP_X0_ZERO) && max_iter > 0;
+        ci.b = b;
+        ci.bdd = bdd;
+        ci.bscale = bscale;
+        ci.tol = rtol;
+        ci.max_iter = max_iter;
+        int rc = GBS_OK;
+        if (!ci.fresh)
+            rc = pcg_setup(ctx, nx, ny, nz, glaw, x, b, mask, u, rtol, max_iter, w, st, setup_flags);
+        else if (!(setup_flags & SETUP_KEEP_DINV))
+            rc = setup_diag(ctx, nx, ny, nz, law, x, mask, w, st);
+        if (rc) return rc;
+        EventPair ev;
+        if (prof) {
+            GBS_CUDA_TRY(ev.create());
+            GBS_CUDA_TRY(cudaEventRecord(ev.e[0], st));
         }
+        rc = chip_run(ctx, &ci, 1, 0, st);
+        if (rc) return rc;
+        if (prof) GBS_CUDA_TRY(cudaEventRecord(ev.e[1], st));
+        if (!out && !prof) return GBS_OK;
+        PcgScalars h;
+        rc = read_scalars(w.sc, &h, st);
+        if (rc) return rc;
+        if (prof) {
+            float ms = 0.0f;
+            GBS_CUDA_TRY(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
+            prof->seconds += 1e-3 * ms;
+            prof->launches += h.iter;
+        }
+        if (out) *out = h;
+        return GBS_OK;
     }
     // from x0 = 0 the one-kernel form starts with a start pass instead of the setup's apply
     // (the persistent kernel keeps the setup: it reads the scalars of iteration 0); only this
@@ -1649,7 +1660,7 @@ int solve_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *l
     const bool dd = use_dd_residual(ctx, o);
     // the residual's element buffer is idle during the inner solves: room for the exchange packets
     const size_t scratch = apply_f64_modal_ws_bytes(nx, ny, nz);
-    const bool chip = chip_ok(ctx, chip_item(nx, ny, nz, pw, w.d32, w.elem, scratch));
+    bool chip = chip_ok(ctx, chip_item(nx, ny, nz, pw, w.d32, w.elem, scratch));
     {
         int rc = outer_start(ctx, nd, u, f, mask, dd, w, st);
         if (rc) return rc;
@@ -1693,25 +1704,27 @@ int solve_run(const gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *l
         }
         // the first round computes 1/diag, later rounds reuse it
         const unsigned flags = SETUP_X0_ZERO | (outer > 1 ? SETUP_KEEP_DINV : 0u);
-        // the fresh start forms b = r / ||r|| itself from the double-float residual
-        const bool scaled_in_start =
-            dd && o->max_iter > total && (chip || fresh_start_ok(ctx, nz, o->fused, o->max_iter - total, flags));
-        if (!scaled_in_start) {
-            rc = outer_scale(ctx, nd, dd, w, st);
-            if (rc) return rc;
-        }
         // Inner tolerance: enough to reach rtol from here, but not below what FP32 resolves.
         double itol = o->rtol / relres;
         if (itol < inner) itol = inner;
         // with the double-float residual the graph loop's publish, finalize and the correction
         // run as one pass (cg_finish_dd_kernel)
         bool finish_left = false;
-        {
+        for (;;) {
+            // the fresh start forms b = r / ||r|| itself from the double-float residual
+            const bool scaled_in_start =
+                dd && o->max_iter > total && (chip || fresh_start_ok(ctx, nz, o->fused, o->max_iter - total, flags));
+            if (!scaled_in_start) {
+                rc = outer_scale(ctx, nd, dd, w, st);
+                if (rc) return rc;
+            }
             NvtxRange range("inner PCG");
             rc = pcg_run(ctx, nx, ny, nz, law, x, w.b32, mask, w.d32, itol, o->max_iter - total, o->check_every, w.pcg,
-                         async ? nullptr : &ps, st, o->profile ? &prof : nullptr, o->fused, flags,
+                         async ? nullptr : &ps, st, chip, o->profile ? &prof : nullptr, o->fused, flags,
                          scaled_in_start ? (const float2 *)w.r64 : nullptr, scaled_in_start ? &w.os->scale : nullptr,
                          dd ? &finish_left : nullptr, w.elem, scratch);
+            if (rc != kChipRefused) break;
+            chip = false;  // for the rest of this solve
         }
         if (rc) return rc;
         if (async) {
@@ -1969,21 +1982,21 @@ extern "C" int gbsimp_time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, co
     GBS_LAUNCH_CHECK("time_pcg_apply setup");
     const ChipItem ci = chip_item(nx, ny, nz, w, xu);
     if (chip_ok(ctx, ci)) {  // `reps` iterations of the on-chip form, its loads and stores included
-        cudaEvent_t e0, e1;
-        GBS_CUDA_TRY(cudaEventCreate(&e0));
-        GBS_CUDA_TRY(cudaEventCreate(&e1));
+        EventPair ev;
         float ms = 0.0f;
+        GBS_CUDA_TRY(ev.create());
         int rc = chip_run(ctx, &ci, 1, reps, st);  // warm-up
-        cudaError_t e = cudaSuccess;
-        if (!rc && (e = cudaEventRecord(e0, st)) == cudaSuccess && !(rc = chip_run(ctx, &ci, 1, reps, st)) &&
-            (e = cudaEventRecord(e1, st)) == cudaSuccess && (e = cudaEventSynchronize(e1)) == cudaSuccess)
-            e = cudaEventElapsedTime(&ms, e0, e1);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        if (rc) return rc;
-        if (e != cudaSuccess) return cuda_error(e, "time_pcg_apply on-chip run");
-        *seconds_per_launch = 1e-3 * ms / reps;
-        return GBS_OK;
+        if (rc == GBS_OK) {
+            GBS_CUDA_TRY(cudaEventRecord(ev.e[0], st));
+            rc = chip_run(ctx, &ci, 1, reps, st);
+        }
+        if (rc == GBS_OK) {
+            GBS_CUDA_TRY(cudaEventRecord(ev.e[1], st));
+            GBS_CUDA_TRY(cudaEventSynchronize(ev.e[1]));
+            GBS_CUDA_TRY(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
+            *seconds_per_launch = 1e-3 * ms / reps;
+        }
+        if (rc != kChipRefused) return rc;
     }
     if (modal) {
         const int r = modal_prepare(ctx, nz);
@@ -2056,8 +2069,11 @@ extern "C" int gbsimp_pcg_f32(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbs
     if ((uintptr_t)u & 15) return set_error(GBS_EINVAL, "gbsimp_pcg_f32: u must be 16-byte aligned");
     PcgScalars h;
     ApplyProfile prof;
-    int rc = pcg_run(ctx, nx, ny, nz, law, x, b, node_mask, u, opts->rtol, opts->max_iter, opts->check_every, ws, &h,
-                     (cudaStream_t)stream, opts->profile ? &prof : nullptr, opts->fused);
+    int rc = kChipRefused;
+    for (const bool chip : {true, false})
+        if (rc == kChipRefused)
+            rc = pcg_run(ctx, nx, ny, nz, law, x, b, node_mask, u, opts->rtol, opts->max_iter, opts->check_every, ws, &h,
+                         (cudaStream_t)stream, chip, opts->profile ? &prof : nullptr, opts->fused);
     if (rc) return rc;
     if (stats) {
         stats->apply_seconds = prof.seconds;
@@ -2345,6 +2361,7 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
         std::vector<ChipItem> ci;
         for (int j : c) ci.push_back(chip_started[j]);
         const int rc = chip_run(ctx, ci.data(), (int)ci.size(), budget, st);
+        if (rc == kChipRefused) return set_error(GBS_EINVAL, "gbsimp_batch: cooperative launch refused");
         if (rc) return rc;
     }
     for (int i : act)

@@ -876,15 +876,20 @@ using ChipKernel = void (*)(const ModalK, unsigned, int, const ChipTable);
 static const ChipKernel chip_kern[5] = {pcg_chip_kernel<1>, pcg_chip_kernel<2>, pcg_chip_kernel<4>, pcg_chip_kernel<5>,
                                         pcg_chip_kernel<kChipQ>};
 
-// Sets the kernels' shared-memory limit once per device; false without cooperative launches.
+// Sets the kernels' shared-memory limit once per device; false without cooperative launches or when a
+// CTA does not fit an SM.
 static bool chip_coop(const gbsimp_ctx *ctx) {
     static std::atomic<int> ready[128];  // every thread stores the same value
     const int dev = ctx->device >= 0 && ctx->device < 128 ? ctx->device : 0;
     if (ready[dev] == 0) {
         int coop = 0;
         bool ok = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop;
-        for (ChipKernel k : chip_kern)
-            ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kChipSmemMax) == cudaSuccess;
+        for (ChipKernel k : chip_kern) {
+            int per_sm = 0;
+            ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kChipSmemMax) == cudaSuccess &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kChipNT, kChipSmemMax) == cudaSuccess &&
+                 per_sm > 0;
+        }
         (void)cudaGetLastError();
         ready[dev] = ok ? 1 : -1;
     }
@@ -942,12 +947,13 @@ static const ChipPlans &chip_plans(const gbsimp_ctx *ctx, const ChipItem &it) {
 int chip_min_blocks(const gbsimp_ctx *ctx, const ChipItem &it) {
     // a cheap bound first: the boxes' nodes cover the grid's
     const int64_t room = (int64_t)std::min(ctx->num_sms, kChipNT) * 2 * kChipNT * kChipQ;
-    if (!ctx->modal_ok || (int64_t)it.nx * it.ny * it.nz > room || !chip_coop(ctx)) return 0;
+    if (!ctx->modal_ok || ctx->diag[GBSIMP_DIAG_CHIP] == 1 || (int64_t)it.nx * it.ny * it.nz > room || !chip_coop(ctx))
+        return 0;
     return chip_plans(ctx, it).least;
 }
 
 int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cudaStream_t st) {
-    if (n <= 0 || n > kChipMaxDesigns || !ctx->modal_ok || !chip_coop(ctx)) return GBS_EINVAL;
+    if (n <= 0 || n > kChipMaxDesigns || !ctx->modal_ok || !chip_coop(ctx)) return kChipRefused;
     const int sms = std::min(ctx->num_sms, kChipNT);
     ChipGeom geo[kChipMaxDesigns] = {};
     auto blocks = [&](int i) { return geo[i].Px * geo[i].Py * geo[i].Pz; };
@@ -957,13 +963,13 @@ int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cu
     int used = 0;
     for (int i = 0; i < n; ++i) {
         const ChipPlans &P = chip_plans(ctx, items[i]);
-        if (P.least == 0) return GBS_EINVAL;
+        if (P.least == 0) return kChipRefused;
         const auto &a = P.at[n == 1 ? sms : P.least];
         geo[i] = a.g;
         cost[i] = a.cost;
         used += blocks(i);
     }
-    if (used > sms) return GBS_EINVAL;
+    if (used > sms) return kChipRefused;
     bool stuck[kChipMaxDesigns] = {};
     while (n > 1) {
         int j = -1;
@@ -1011,10 +1017,12 @@ int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cu
     unsigned polls = wait_polls(ctx);
     void *args[] = {&km, &polls, &budget, &T};
     const cudaError_t e =
-        cudaLaunchCooperativeKernel((const void *)chip_kern[v], dim3((unsigned)block0), dim3(kChipNT), args, smem, st);
+        ctx->diag[GBSIMP_DIAG_CHIP] == 2
+            ? cudaErrorCooperativeLaunchTooLarge
+            : cudaLaunchCooperativeKernel((const void *)chip_kern[v], dim3((unsigned)block0), dim3(kChipNT), args, smem, st);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        return set_error(GBS_EINVAL, "cooperative launch refused: %s", cudaGetErrorString(e));
+        return kChipRefused;
     }
     count_launches(1);
     return GBS_OK;

@@ -44,7 +44,9 @@ struct ChipItem {
 int chip_min_blocks(const gbsimp_ctx *ctx, const ChipItem &it);
 // Runs the inner PCGs of n designs in one cooperative launch, CTAs shared so that the designs'
 // modelled iteration times even out: at most `budget` iterations each (0: to the end). Returns
-// GBS_EINVAL without launching when they do not fit together.
+// kChipRefused, with nothing run, when they do not fit together or the launch is refused (a context
+// that may use fewer SMs than the device has, for instance): the caller takes a streaming form.
+constexpr int kChipRefused = -1;
 int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cudaStream_t st);
 
 }  // namespace gbs

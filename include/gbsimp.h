@@ -371,8 +371,10 @@ int gbsimp_barrier_selftest(gbsimp_ctx *ctx, int extra_arrivals, double wait_sec
 /* Diagnostics of one context, for tests (no counterpart in the reference). A negative value, the
  * default, switches a key off. Not to be set while a call on the context is running.
  * GBSIMP_DIAG_TIMEOUT: 0: the waits of the on-chip PCG and of the OC update for other blocks run out
- * after one look; b > 0: block b of an on-chip PCG reports a wait that ran out at its end. */
-enum { GBSIMP_DIAG_TIMEOUT = 1 };
+ * after one look; b > 0: block b of an on-chip PCG reports a wait that ran out at its end.
+ * GBSIMP_DIAG_CHIP: 0: the chip holds no grid, so that every solve runs in its streaming form; 1: the
+ * on-chip PCG's cooperative launches are taken for refused. */
+enum { GBSIMP_DIAG_TIMEOUT = 1, GBSIMP_DIAG_CHIP = 2 };
 int gbsimp_set_diagnostic(gbsimp_ctx *ctx, int key, int64_t value);
 
 /* ---- reductions used by the host loops -------------------------------------------- */
