@@ -2278,18 +2278,31 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
     std::vector<int> fresh;
     for (int i : res)
         if (items[i].state == 0) fresh.push_back(i);
-    // Grids that fit the chip run in the on-chip form, started or resumed; the others as below.
+    const int group = o->batch_group > 0 && o->batch_group < kMaxFused ? o->batch_group : kMaxFused;
+    const int share = o->batch_share == 1 ? 1 : 0;
+    // Grids that fit the chip run in the on-chip form, started or resumed; the others as below, those of
+    // a refused launch among them (a paused one starts its inner solve again: its residual is still in
+    // the workspace).
     auto citem = [&](int i) {
         gbsimp_batch_item &it = items[i];
         SolveWs w = solve_ws(it.ws, it.nx, it.ny, it.nz);
         return chip_item(it.nx, it.ny, it.nz, pcg_ws(w.pcg, it.nx, it.ny, it.nz), w.d32, w.elem,
                          apply_f64_modal_ws_bytes(it.nx, it.ny, it.nz));
     };
-    std::vector<int> chip_items;
+    auto anew = [&](int i) {
+        items[i].stats.inner_active = 0;
+        items[i].stats.inner_iters = 0;
+        fresh.push_back(i);
+    };
+    std::vector<int> chip_try, chip_items;
     std::vector<ChipItem> chip_started;
     for (int i : act)
-        if (items[i].state == 0 && items[i].stats.inner_active == 1 && chip_ok(ctx, citem(i))) {
-            chip_items.push_back(i);
+        if (items[i].state == 0 && items[i].stats.inner_active == 3) {
+            if (!chip_ok(ctx, citem(i))) {
+                anew(i);
+                continue;
+            }
+            chip_try.push_back(i);
             chip_started.push_back(citem(i));
         }
     {
@@ -2318,10 +2331,20 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
             }
             ci.tol = itol;
             ci.max_iter = o->max_iter - it.stats.iterations;
-            chip_items.push_back(i);
+            chip_try.push_back(i);
             chip_started.push_back(ci);
         }
         fresh.swap(other);
+    }
+    for (const std::vector<int> &c : chip_groups(ctx, chip_started, o->fused ? std::min(group, kChipMaxDesigns) : 1)) {
+        std::vector<ChipItem> ci;
+        for (int j : c) ci.push_back(chip_started[j]);
+        const int rc = chip_run(ctx, ci.data(), (int)ci.size(), budget, st);
+        if (rc && rc != kChipRefused) return rc;
+        for (int j : c) {
+            if (rc) anew(chip_try[j]);
+            else chip_items.push_back(chip_try[j]);
+        }
     }
     for (int i : fresh) {
         gbsimp_batch_item &it = items[i];
@@ -2337,16 +2360,14 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
         if (rc) return rc;
     }
     // ---- run the inner PCGs: paused persistent solves, then the new ones ---------------------
-    // A paused solve resumes in the form it started in (the persistent kernel and the graph loop
-    // keep their scalars differently). New solves are packed greedily into persistent launches
-    // of designs that are resident together; one that fits no launch runs its own graph loop.
+    // A paused solve resumes in the form it started in (the forms keep their state differently). New
+    // solves are packed greedily into persistent launches of designs that are resident together; one
+    // that fits no launch runs its own graph loop.
     auto fitem = [&](int i) {
         gbsimp_batch_item &it = items[i];
         SolveWs w = solve_ws(it.ws, it.nx, it.ny, it.nz);
         return FusedItem{it.nx, it.ny, it.nz, it.x, it.node_mask, w.d32, pcg_ws(w.pcg, it.nx, it.ny, it.nz)};
     };
-    const int group = o->batch_group > 0 && o->batch_group < kMaxFused ? o->batch_group : kMaxFused;
-    const int share = o->batch_share == 1 ? 1 : 0;
     auto fits = [&](const std::vector<int> &c) {
         if (c.empty() || c.size() > (size_t)group) return false;
         FusedItem fi[kMaxFused];
@@ -2357,15 +2378,8 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
     std::vector<int> order, graph_items;
     std::vector<char> on_chip(n, 0);
     for (int i : chip_items) on_chip[i] = 1;
-    for (const std::vector<int> &c : chip_groups(ctx, chip_started, o->fused ? std::min(group, kChipMaxDesigns) : 1)) {
-        std::vector<ChipItem> ci;
-        for (int j : c) ci.push_back(chip_started[j]);
-        const int rc = chip_run(ctx, ci.data(), (int)ci.size(), budget, st);
-        if (rc == kChipRefused) return set_error(GBS_EINVAL, "gbsimp_batch: cooperative launch refused");
-        if (rc) return rc;
-    }
     for (int i : act)
-        if (items[i].state == 0 && items[i].stats.inner_active == 1 && !on_chip[i]) order.push_back(i);
+        if (items[i].state == 0 && items[i].stats.inner_active == 1) order.push_back(i);
     for (int i : act)
         if (items[i].state == 0 && items[i].stats.inner_active == 2) graph_items.push_back(i);
     for (int i : fresh) {
@@ -2454,7 +2468,7 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
             it.stats.iterations += h.iter - it.stats.inner_iters;
             if (!h.done) {  // paused by the budget: resumes next round, in the same form
                 it.stats.inner_iters = h.iter;
-                it.stats.inner_active = graph_loop ? 2 : 1;
+                it.stats.inner_active = on_chip[inn[k + j]] ? 3 : (graph_loop ? 2 : 1);
                 continue;
             }
             it.stats.inner_iters = 0;
@@ -2488,7 +2502,7 @@ static int check_batch(gbsimp_ctx *ctx, gbsimp_batch_item *items, int n, const g
             return set_error(GBS_EINVAL, "gbsimp_batch: item %d has bad arguments", i);
         if (it.ws_bytes < solve_ws_bytes_impl(it.nx, it.ny, it.nz))
             return set_error(GBS_EINVAL, "gbsimp_batch: item %d workspace too small", i);
-        if (it.stats.inner_active < 0 || it.stats.inner_active > 2 || it.stats.inner_iters < 0)
+        if (it.stats.inner_active < 0 || it.stats.inner_active > 3 || it.stats.inner_iters < 0)
             return set_error(GBS_EINVAL, "gbsimp_batch: item %d has library-owned stats fields set (zero its stats)", i);
     }
     return GBS_OK;

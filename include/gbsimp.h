@@ -97,8 +97,8 @@ typedef struct gbsimp_solve_stats {
     int32_t status;       /* GBS_OK, GBS_ENOTCONV, GBS_EBREAKDOWN, GBS_ENONFINITE, GBS_ETIMEOUT */
     int32_t iterations;   /* FP32 PCG iterations (all outer corrections together) */
     int32_t outer;        /* outer residual evaluations */
-    int32_t inner_active; /* batched rounds (library-owned, start at 0): 1 or 2 while an inner
-                             PCG is paused by the round budget (persistent kernel / graph loop) */
+    int32_t inner_active; /* batched rounds (library-owned, start at 0): 1, 2 or 3 while an inner PCG is
+                             paused by the round budget (persistent kernel / graph loop / on chip) */
     double relres;        /* last ||D(f - K u)|| / ||D f|| */
     double seconds;       /* host wall time of the call */
     double apply_seconds; /* device time of the PCG apply launches (opts->profile only) */
