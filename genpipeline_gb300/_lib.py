@@ -81,6 +81,7 @@ class SimpOpts(C.Structure):
 
 DIAG_TIMEOUT = 1
 DIAG_CHIP = 2
+DIAG_OC = 3
 
 _P = C.c_void_p
 _I = C.c_int

@@ -434,7 +434,7 @@ struct gbsimp_ctx {
     gbs::ModalKD kmd;       // the same in FP64
     unsigned ke_version;    // bumped by every set_ke (keys the graph cache)
     void *graphs;           // gbs::GraphCache* (pcg.cu): instantiated device-loop graphs
-    int64_t diag[3];        // gbsimp_set_diagnostic, by key: the value + 1, 0 where the default holds
+    int64_t diag[4];        // gbsimp_set_diagnostic, by key: the value + 1, 0 where the default holds
 };
 
 namespace gbs {

@@ -1096,10 +1096,12 @@ static int oc_coop_blocks(const gbsimp_ctx *ctx) {
     if (dev < 0 || dev >= 64) return 0;
     int v = cache[dev].load(std::memory_order_relaxed);
     if (v != 0) return v > 0 ? v : 0;
-    int coop = 0;
+    int coop = 0, per_sm = 0;
     const int most = (int)(kCoopSums + 3 * sizeof(float) * kCoopThreads * kCoopKeep);
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-        cudaFuncSetAttribute(oc_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) {
+        cudaFuncSetAttribute(oc_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, oc_coop_kernel, kCoopThreads, most) != cudaSuccess ||
+        per_sm < 1) {
         (void)cudaGetLastError();
         cache[dev].store(-1, std::memory_order_relaxed);
         return 0;
@@ -1137,12 +1139,19 @@ int oc_run_impl(const gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin, cons
         unsigned polls = wait_polls(ctx);
         void *args[] = {(void *)&n, (void *)&P, (void *)&x, (void *)&dc, (void *)&preserved, (void *)&w.w,
                         (void *)&box, (void *)&w.sc, (void *)&xnew, (void *)&keep, (void *)&polls};
-        GBS_CUDA_TRY(cudaLaunchCooperativeKernel((void *)oc_coop_kernel, dim3((unsigned)nb), dim3(kCoopThreads), args,
-                                                 kCoopSums + 3 * sizeof(float) * keep, st));
-        GBS_LAUNCH_CHECK("oc_coop_kernel");
-        return filter_launch(ctx, nx, ny, nz, rmin, 0, w.hs, xnew, preserved, xphys, st);
+        const cudaError_t e =
+            ctx->diag[GBSIMP_DIAG_OC] == 1
+                ? cudaErrorCooperativeLaunchTooLarge
+                : cudaLaunchCooperativeKernel((void *)oc_coop_kernel, dim3((unsigned)nb), dim3(kCoopThreads), args,
+                                              kCoopSums + 3 * sizeof(float) * keep, st);
+        if (e == cudaSuccess) {
+            GBS_LAUNCH_CHECK("oc_coop_kernel");
+            return filter_launch(ctx, nx, ny, nz, rmin, 0, w.hs, xnew, preserved, xphys, st);
+        }
+        // refused: a context that may use fewer SMs than the device has, say, does not hold a block per SM
+        (void)cudaGetLastError();
     }
-    // kOcNodes double-float partials per block fit the 4 * 4096 doubles of the workspace
+    // a launch per round; kOcNodes double-float partials per block fit the 4 * 4096 doubles of the workspace
     int64_t mb = (n + kOcThreads - 1) / kOcThreads;
     const int64_t mcap = 2LL * (ctx->num_sms > 0 ? ctx->num_sms : 148);
     mb = mb > mcap ? mcap : (mb < 1 ? 1 : mb);

@@ -373,8 +373,9 @@ int gbsimp_barrier_selftest(gbsimp_ctx *ctx, int extra_arrivals, double wait_sec
  * GBSIMP_DIAG_TIMEOUT: 0: the waits of the on-chip PCG and of the OC update for other blocks run out
  * after one look; b > 0: block b of an on-chip PCG reports a wait that ran out at its end.
  * GBSIMP_DIAG_CHIP: 0: the chip holds no grid, so that every solve runs in its streaming form; 1: the
- * on-chip PCG's cooperative launches are taken for refused. */
-enum { GBSIMP_DIAG_TIMEOUT = 1, GBSIMP_DIAG_CHIP = 2 };
+ * on-chip PCG's cooperative launches are taken for refused.
+ * GBSIMP_DIAG_OC: 0: the OC update's cooperative launch is taken for refused. */
+enum { GBSIMP_DIAG_TIMEOUT = 1, GBSIMP_DIAG_CHIP = 2, GBSIMP_DIAG_OC = 3 };
 int gbsimp_set_diagnostic(gbsimp_ctx *ctx, int key, int64_t value);
 
 /* ---- reductions used by the host loops -------------------------------------------- */
