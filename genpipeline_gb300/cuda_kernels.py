@@ -33,7 +33,9 @@ def _engine_for(Ke: torch.Tensor, device: torch.device) -> Engine:
     pageable copy and a digest."""
     buf = getattr(_STAGE, "ke", None)
     if buf is None:
-        buf = _STAGE.ke = torch.empty(576, dtype=torch.float64, pin_memory=True)
+        # a host tensor to be written on any later call, whatever modes this one runs in
+        with torch.inference_mode(False):
+            buf = _STAGE.ke = torch.empty(576, dtype=torch.float64, device="cpu", pin_memory=True)
     buf.copy_(Ke.detach().reshape(576), non_blocking=True)
     if Ke.is_cuda:
         torch.cuda.current_stream(Ke.device).synchronize()
