@@ -1,4 +1,6 @@
 // apply.cu -- C-ABI entry points of the element stiffness apply y = D K(x) D p.
+#include <float.h>
+
 #include "apply_modal.cuh"
 #include "internal.h"
 
@@ -81,8 +83,10 @@ __global__ void __launch_bounds__(kEdofNT) apply_edof_kernel(int64_t n_elem, int
 }
 
 // The energy's 24 products, exact to their rounding errors, are summed in FP32 pairs (2^-46); an FP64 sum,
-// with its conversions, took half of the kernel's 16 us at 65536 elements (6.1 so). Where a pair does not
-// hold the sum (infinities, NaN, energies below the normal range) it runs in FP64.
+// with its conversions, took half of the kernel's 16 us at 65536 elements (6.1 so). The displacements are
+// scaled by a power of two to a largest component between 1 and 2, so that displacements of any size keep
+// to the pairs (at 1e-13 and below the sums ran in FP64 and the kernel took 10.7 us). Where a pair does not hold the
+// sum all the same (infinities, NaN, a stiffness near either end of the range) it runs in FP64.
 template <typename I>
 __global__ void __launch_bounds__(kEdofNT) sens_edof_kernel(int64_t n_elem, int64_t n_dof, const void *edof,
                                                             Law<float> law, const KeF ke, const float *x,
@@ -98,7 +102,12 @@ __global__ void __launch_bounds__(kEdofNT) sens_edof_kernel(int64_t n_elem, int6
         ue[q] = (d >= 0 && d < n_dof) ? u[d] : 0.0f;
         most = fmaxf(most, fabsf(ue[q]));
     }
-    float h = 0.0f, l = 0.0f;
+    // the exponent of the largest component; 2^-ex as a product of two factors within the range
+    const int ex = most > 0.0f && most <= FLT_MAX ? ilogbf(most) : 0;
+    const float f1 = __int_as_float((127 - ex / 2) << 23), f2 = __int_as_float((127 - (ex - ex / 2)) << 23);
+    float h = 0.0f, l = 0.0f, ws = 0.0f, ss = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 24; ++q) ue[q] = ue[q] * f1 * f2;
 #pragma unroll
     for (int r = 0; r < 24; ++r) {
         float s = 0.0f;
@@ -109,9 +118,11 @@ __global__ void __launch_bounds__(kEdofNT) sens_edof_kernel(int64_t n_elem, int6
         l = __fadd_rn(l, __fmaf_rn(ue[r], s, -w));
         two_sum(h, w, h, d);
         l = __fadd_rn(l, d);
+        ws = fmaxf(ws, fabsf(w));
+        ss = fmaxf(ss, fabsf(s));
     }
     float ce = h + l;
-    if (!(fabsf(ce) < 1e37f) || (most > 0.0f && fabsf(ce) < 1e-25f)) {
+    if (!(fabsf(ce) < 1e37f) || (ss > 0.0f && ws < 1e-25f)) {
         double c = 0.0;
 #pragma unroll 1
         for (int r = 0; r < 24; ++r) {
@@ -125,6 +136,8 @@ __global__ void __launch_bounds__(kEdofNT) sens_edof_kernel(int64_t n_elem, int6
             c += (double)ur * (double)s;
         }
         ce = (float)c;
+    } else if (ex != 0) {
+        ce = ldexpf(ce, 2 * ex);
     }
     dc[e] = -dmodulus(law, x[e]) * ce;
 }

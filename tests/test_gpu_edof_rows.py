@@ -45,3 +45,19 @@ def test_energies_outside_the_range_of_a_pair():
     np.testing.assert_allclose(dc[1], -24 * 9e36, rtol=1e-6)
     assert not np.isfinite(dc[2])
     np.testing.assert_allclose(dc[3], -24.0, rtol=1e-6)
+
+
+@pytest.mark.parametrize("k", [-50, -45, -10, 15, 50])
+def test_energies_scale_with_the_square_of_the_displacements(k):
+    """A power of two in u is its square in the energy, to the last bit (energies from 1 to 1e4 here, so
+    that FP32 holds both)."""
+    rng = np.random.default_rng(2)
+    n, nd = 300, 400
+    R = rng.standard_normal((24, 24))
+    K = torch.as_tensor((R @ R.T).astype(np.float32), device="cuda")
+    edof = torch.as_tensor(rng.integers(0, nd, (n, 24)), device="cuda")
+    x = torch.as_tensor(rng.uniform(0.5, 1, n).astype(np.float32), device="cuda")
+    u = torch.as_tensor(rng.standard_normal(nd).astype(np.float32), device="cuda")
+    want = cuda_kernels.simp_sensitivity(x, u, K, edof, 3.0, n, 1, 1)
+    got = cuda_kernels.simp_sensitivity(x, u * 2.0 ** k, K, edof, 3.0, n, 1, 1) * 2.0 ** -k * 2.0 ** -k
+    assert torch.equal(got, want)
