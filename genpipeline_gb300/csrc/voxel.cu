@@ -113,9 +113,11 @@ __device__ __forceinline__ void vox_add(float2 w, float v, float &s, float &e) {
     e = __fadd_rn(e, d);
 }
 
-// What the pair s + e cannot hold (an infinity or NaN among the inputs, an overflow on the way, a sum
-// whose errors fall below the FP32 range) is summed again in FP64, without the taps of weight zero.
-__device__ __forceinline__ bool vox_plain(float s) { return s == 0.0f || (fabsf(s) > 1e-30f && fabsf(s) < 1e38f); }
+// What the pair s + e cannot hold (an infinity or NaN among the inputs, an overflow on the way) is summed
+// again in FP64, without the taps of weight zero. A sum so small that its errors fall below the FP32 range
+// stays: the logistic takes 1/2 from every sum, beside which it is nothing to FP64 either. (Summed again,
+// a void of 1e-35 took 567 us where 16 x 64^3 -> 32^3 of ordinary values takes 52.)
+__device__ __forceinline__ bool vox_plain(float s) { return fabsf(s) < 1e38f; }
 static __device__ __noinline__ double vox_sum64(const VoxRow *R, const float *src, long long stride) {
     double acc = 0.0;
     for (int k = 0; k < R->count; ++k) {

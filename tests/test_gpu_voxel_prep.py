@@ -37,3 +37,15 @@ def test_values_outside_the_range_of_a_pair():
     one[0, 0, 0] = np.nan
     got = get_engine().voxel_prep(torch.from_numpy(one).cuda(), (4, 4, 4), 0.3, 15.0).cpu().numpy()
     assert np.isnan(got).sum() == 8 and np.isnan(got[:2, :2, :2]).all()  # radius one, mirrored at the border
+
+
+@pytest.mark.parametrize("void", [1e-29, 1e-32, 1e-38, 1e-44])
+@pytest.mark.parametrize("shape,out", [((5, 33, 64), (3, 17, 32)), ((40, 3, 65), (20, 2, 33))])
+def test_a_void_of_small_values(shape, out, void):
+    """Solids in a void at the low end of the FP32 range, as a steep decoder leaves it."""
+    rng = np.random.default_rng(3)
+    vol = np.where(rng.random(shape) < 0.5, rng.random(shape), void * rng.random(shape)).astype(np.float32)
+    vol[: shape[0] // 2] = void
+    got = get_engine().voxel_prep(torch.from_numpy(vol).cuda(), out).cpu().numpy()
+    # as above: two FP32 roundings through a slope of 15 / 4, and the last one
+    assert np.abs(got - V.voxel_prep(vol, out)).max() <= 2 * 2.0 ** -25 * 15 / 4 + 2.0 ** -24
