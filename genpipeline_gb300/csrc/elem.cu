@@ -173,8 +173,10 @@ constexpr int kMaxStencil = 1024;
 struct Stencil {
     int n;
     int r;
+    int flat;              // 1: doff[] holds the flat offsets of this grid
     int off[kMaxStencil];  // dx, dy, dz packed as signed bytes
     float w[kMaxStencil];  // rmin - dist > 0
+    int doff[kMaxStencil]; // (dx ny + dy) nz + dz: the element offset in x-y-z order
 };
 
 // The neighbourhood of simp_solver.py:1553-1565: offsets of the box of half-width
@@ -184,6 +186,7 @@ static int make_stencil(double rmin, Stencil *s) {
     const int r = (int)ceil(rmin);
     s->n = 0;
     s->r = r;
+    s->flat = 0;
     for (int di = -r; di <= r; ++di)
         for (int dj = -r; dj <= r; ++dj)
             for (int dk = -r; dk <= r; ++dk) {
@@ -198,6 +201,25 @@ static int make_stencil(double rmin, Stencil *s) {
                 ++s->n;
             }
     return GBS_OK;
+}
+
+// The flat element offsets of the stencil for a grid of ny x nz element rows, when every
+// one fits in an int (s->flat = 1; otherwise the kernel uses the bounds-checked path only).
+static void set_flat_offsets(int ny, int nz, Stencil *s) {
+    const int64_t reach = (int64_t)s->r * ((int64_t)ny * nz + nz + 1);
+    s->flat = reach < INT32_MAX ? 1 : 0;
+    if (!s->flat) return;
+    for (int q = 0; q < s->n; ++q) {
+        const int o = s->off[q];
+        const int di = (int)(int8_t)(o & 0xff), dj = (int)(int8_t)((o >> 8) & 0xff), dk = (int)(int8_t)((o >> 16) & 0xff);
+        s->doff[q] = (int)(((int64_t)di * ny + dj) * nz + dk);
+    }
+}
+
+__device__ __forceinline__ void neumaier_add(float &s, float &c, float v) {
+    const float t = s + v;
+    c += fabsf(s) >= fabsf(v) ? (s - t) + v : (v - t) + s;
+    s = t;
 }
 
 __device__ __forceinline__ void unpack_off(int o, int &di, int &dj, int &dk) {
@@ -230,8 +252,9 @@ static int filter_columns(const Stencil &st, FilterCols *F) {
     memset(F, 0, sizeof *F);
     for (int h = 0; h <= kFilterR; ++h) {
         F->start[h] = n;
-        for (int i = 0; i <= 2 * kFilterR; ++i)
-            for (int j = 0; j <= 2 * kFilterR; ++j) {
+        if (h > R) continue;
+        for (int i = kFilterR - R; i <= kFilterR + R; ++i)
+            for (int j = kFilterR - R; j <= kFilterR + R; ++j) {
                 if (half[i][j] != h) continue;
                 F->di[n] = (short)(i - kFilterR);
                 F->dj[n] = (short)(j - kFilterR);
@@ -246,6 +269,7 @@ static int filter_columns(const Stencil &st, FilterCols *F) {
 // A block's tile of outputs: ti x tj rows of kt threads, four elements along z each.
 struct FilterTile {
     int ti, tj, kt, nbj, nbk;
+    FastDiv fk, fj;  // by the tile's words per row and rows per plane, margins included
 };
 
 // s + c += the columns of half-extent H and above of the four elements whose window starts at t.
@@ -281,11 +305,68 @@ __device__ __forceinline__ void filter_cols(const FilterCols &F, const float *t,
 
 // mode 0: out = (sum w v) / hs[e] (hs nullable: computed);  mode 1: out = sum w v/hs[e2];
 // mode 2 (hs): out = sum w over in-bounds neighbours. preserved (mode 0): out = 1 there.
-// FP32 products summed with their rounding errors (a few ulp whatever the stencil, up to ~900 terms at
-// rmin 6). Bound by FP32 issue, eight operations per tap. v, v/hs or one (zero outside the grid) of the
-// tile and its margin R goes to shared memory once, and a thread takes four elements along z, so that a
-// column of taps costs it two or three 16-byte loads. A bounds test, a global load, the division and the
-// sum of weights (wanted or not) at every tap took 209 us at 192x96x96 with rmin 3 where this takes 69.
+// A tap at a time, an element per thread, for small work (filter_tiled): nothing to load first, and a
+// tap outside the grid costs its test only. FP32 products summed with their rounding errors (a few ulp
+// whatever the stencil, up to ~900 terms at rmin 6).
+__global__ void __launch_bounds__(256) filter_taps_kernel(int nx, int ny, int nz, const FastDiv fy, const FastDiv fz,
+                                                     const Stencil st, int mode,
+                                                     const float *__restrict__ hs, const float *__restrict__ in,
+                                                     const uint8_t *__restrict__ preserved, float *out) {
+    const int64_t n_elem = (int64_t)nx * ny * nz;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_elem; e += (int64_t)gridDim.x * blockDim.x) {
+        int i, j, k;
+        unflatten3((uint32_t)e, fy, fz, i, j, k);
+        // FP32 with compensated (Neumaier) summation in the fixed stencil order: error of a
+        // few ulp whatever the stencil size (up to ~900 terms at rmin 6).
+        float s = 0.0f, sc = 0.0f, ws = 0.0f, wc = 0.0f;
+        // Away from the x and y faces only z can leave the grid: the same terms in the same
+        // order, with one z test and a precomputed flat offset per term (a warp's elements
+        // lie in one or two z columns, so the branch rarely splits a warp).
+        if (st.flat && i >= st.r && i < nx - st.r && j >= st.r && j < ny - st.r) {
+            for (int q = 0; q < st.n; ++q) {
+                const int k2 = k + (int)(int8_t)((st.off[q] >> 16) & 0xff);
+                if (k2 < 0 || k2 >= nz) continue;
+                const int64_t e2 = e + st.doff[q];
+                const float w = st.w[q];
+                neumaier_add(ws, wc, w);
+                if (mode == 0) neumaier_add(s, sc, w * in[e2]);
+                else if (mode == 1) neumaier_add(s, sc, w * (in[e2] / hs[e2]));
+            }
+        } else {
+            for (int q = 0; q < st.n; ++q) {
+                int di, dj, dk;
+                unpack_off(st.off[q], di, dj, dk);
+                const int i2 = i + di, j2 = j + dj, k2 = k + dk;
+                if (i2 < 0 || i2 >= nx || j2 < 0 || j2 >= ny || k2 < 0 || k2 >= nz) continue;
+                const int64_t e2 = ((int64_t)i2 * ny + j2) * nz + k2;
+                const float w = st.w[q];
+                neumaier_add(ws, wc, w);
+                if (mode == 0) neumaier_add(s, sc, w * in[e2]);
+                else if (mode == 1) neumaier_add(s, sc, w * (in[e2] / hs[e2]));
+            }
+        }
+        s += sc;
+        ws += wc;
+        float o;
+        if (mode == 0) {
+            const float h = hs ? hs[e] : ws;
+            o = s / h;
+            if (preserved && preserved[e]) o = 1.0f;
+        } else if (mode == 1) {
+            o = (float)s;
+        } else {
+            o = (float)ws;
+        }
+        out[e] = o;
+    }
+}
+
+// The same from a tile. FP32 products summed with their rounding errors. Bound by FP32 issue, eight
+// operations per tap. v, v/hs or one (zero outside the grid) of the tile and its margin R goes to shared
+// memory once, and a thread takes four elements along z, so that a column of taps costs it two or three
+// 16-byte loads: 192x96x96 takes 58 us with rmin 3 where a tap at a time takes 173 (device time; rmin
+// 1.5: 22 for 41). The tile's words are dealt to the threads one by one, eight loads in flight each; a warp
+// per row left most lanes idle where rows are short and took 11.0 us at 32x8x8 with rmin 1.5, 5.4 so.
 // Plain FP32 sums along a column would take a third of the operations, but moved the compliance of a
 // twelve-step SIMP run at 20x8x8 by 7e-6.
 template <int R>
@@ -298,28 +379,23 @@ __global__ void __launch_bounds__(256) filter_kernel(int nx, int ny, int nz, con
     const int SK = (4 * T.kt + 2 * R + 3) & ~3, SJ = T.tj + 2 * R, rows = (T.ti + 2 * R) * SJ;
     const int bk = blockIdx.x % T.nbk, bij = blockIdx.x / T.nbk, bj = bij % T.nbj, bi = bij / T.nbj;
     const int i0 = bi * T.ti, j0 = bj * T.tj, k0 = bk * 4 * T.kt;
-    const int tid = threadIdx.x, lane = tid & 31, kt = tid % T.kt, ij = tid / T.kt, jl = ij % T.tj, il = ij / T.tj;
+    const int tid = threadIdx.x, kt = tid % T.kt, ij = tid / T.kt, jl = ij % T.tj, il = ij / T.tj;
     float s[4], c[4], h[4] = {1.0f, 1.0f, 1.0f, 1.0f};
     const bool own = mode == 0 && hs == nullptr;  // the sums of weights first
     for (int pass = own ? 0 : 1; pass < 2; ++pass) {
         const bool ones = mode == 2 || pass == 0;
-#pragma unroll 4
-        for (int r = tid >> 5; r < rows; r += (int)blockDim.x >> 5) {
-            const int a = r / SJ, i = i0 + a - R, j = j0 + (r - a * SJ) - R;
-            const bool in_ij = i >= 0 && i < nx && j >= 0 && j < ny;
-            const int64_t e = ((int64_t)i * ny + j) * nz;
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const int kk = lane + 32 * p, k = k0 + kk - R;
-                if (kk >= SK) continue;
-                float v = 0.0f;
-                if (in_ij && k >= 0 && k < nz) {
-                    if (ones) v = 1.0f;
-                    else if (mode == 1) v = in[e + k] / hs[e + k];
-                    else v = in[e + k];
-                }
-                tile[r * SK + kk] = v;
+#pragma unroll 8
+        for (int q = tid; q < rows * SK; q += blockDim.x) {
+            const int r = (int)fdiv((uint32_t)q, T.fk), a = (int)fdiv((uint32_t)r, T.fj);
+            const int i = i0 + a - R, j = j0 + (r - a * SJ) - R, k = k0 + (q - r * SK) - R;
+            float v = 0.0f;
+            if (i >= 0 && i < nx && j >= 0 && j < ny && k >= 0 && k < nz) {
+                const int64_t e = ((int64_t)i * ny + j) * nz + k;
+                if (ones) v = 1.0f;
+                else if (mode == 1) v = in[e] / hs[e];
+                else v = in[e];
             }
+            tile[q] = v;
         }
         __syncthreads();
 #pragma unroll
@@ -364,7 +440,7 @@ static unsigned elem_blocks(const gbsimp_ctx *ctx, int64_t n, int threads) {
 // larger would leave SMs without one.
 static FilterTile filter_tile(const gbsimp_ctx *ctx, int nx, int ny, int nz, int R, int *threads) {
     auto up = [](int a, int b) { return (a + b - 1) / b; };
-    FilterTile T{1, 1, 1, 1, 1};
+    FilterTile T{1, 1, 1, 1, 1, {}, {}};
     while (T.kt < 8 && 4 * T.kt < nz) T.kt *= 2;
     T.nbk = up(nz, 4 * T.kt);
     const int sms = ctx->num_sms > 0 ? ctx->num_sms : 148;
@@ -383,7 +459,26 @@ static FilterTile filter_tile(const gbsimp_ctx *ctx, int nx, int ny, int nz, int
         T.nbj = up(ny, T.tj);
         if ((int64_t)up(nx, T.ti) * T.nbj * T.nbk >= sms) break;
     }
+    T.fk = fast_div((uint32_t)((4 * T.kt + 2 * R + 3) & ~3));
+    T.fj = fast_div((uint32_t)(T.tj + 2 * R));
     return T;
+}
+
+// Whether the tiled kernel takes the call. Device times, a tap at a time -> tiled, at the lines: seven
+// taps (rmin up to sqrt 2) 48^3 3.7 -> 5.2 us, 256x256x100 67 -> 81; 19 taps 32^3 5.0 -> 6.2, 33^3
+// 6.4 -> 5.8, 32x8x8 6.6 -> 5.4 but 3x60x60 5.1 -> 6.6; 81 taps 32^3 13.6 -> 12.0, 1x64x64 7.8 -> 9.5,
+// 1x450x450 20.5 -> 13.0, 1x1x200000 17 -> 164 (the columns beyond the grid are all zeros); 93 taps
+// 450x450x1 27 -> 34 (three of a thread's four elements lie outside); 895 taps 1x450x450 174 -> 203.
+// With the sums of weights to form as well (own), which the tile does one after the other: 81 taps 32^3
+// 13.5 -> 17.7, 33^3 21.0 -> 16.0, 19 taps 64^3 9.4 -> 8.9, 256x256x100 142 -> 153, 895 taps 2x300x300
+// 171 -> 207.
+static bool filter_tiled(int nx, int ny, int nz, int taps, bool own) {
+    const int64_t n = (int64_t)nx * ny * nz;
+    const int lo = std::min(nx, std::min(ny, nz)), hi = std::max(nx, std::max(ny, nz));
+    if (taps <= 7) return false;
+    if (lo == 1) return !own && taps >= 60 && taps < 800 && n >= 100000 && n / hi >= 32 && nz >= 32;
+    if (own) return taps >= 60 && n > 33000 && lo > 2;
+    return taps >= 60 || n > 33000 || (nz < 16 && lo > 3);
 }
 
 int filter_launch(const gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin, int mode, const float *hs,
@@ -391,6 +486,14 @@ int filter_launch(const gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin, in
     Stencil s;
     int rc = make_stencil(rmin, &s);
     if (rc) return rc;
+    if (!filter_tiled(nx, ny, nz, s.n, mode == 0 && !hs)) {
+        const int64_t n = (int64_t)nx * ny * nz;
+        set_flat_offsets(ny, nz, &s);
+        filter_taps_kernel<<<elem_blocks(ctx, n, 256), 256, 0, st>>>(nx, ny, nz, fast_div(ny), fast_div(nz), s, mode, hs,
+                                                                     in, preserved, out);
+        GBS_LAUNCH_CHECK("filter_taps_kernel");
+        return GBS_OK;
+    }
     FilterCols F;
     const int R = filter_columns(s, &F);
     int nt = 256;
