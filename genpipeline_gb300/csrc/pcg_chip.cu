@@ -826,14 +826,14 @@ __global__ void __launch_bounds__(kChipNT, 1)
 
 // ---- plans ------------------------------------------------------------------------------------
 // Modelled SM cycles of one iteration of a box, fitted to clock counts of its phases over boxes of
-// 2x8x8 to 16x8x16 elements (within 10 %): the march's steps, dearer with a second warp on a
-// scheduler and with several slabs of rows longer than four (their planes meet in shared memory's
-// banks); the update of q places per thread; the block's sums; the exchange; and what the widest
+// 2x8x8 to 16x8x16 elements (within 10 %; over 190 grids 0.78 to 1.19 of it): the march's steps,
+// dearer with a second warp on a scheduler and with several slabs (their planes meet in shared memory's
+// banks; not in single steps of rows up to four); the update of q places per thread; the block's sums; the exchange; and what the widest
 // kernel, whose iteration outgrows the instruction cache, takes longer.
 static double chip_cost(int ex, int ez, int q, int warps, int G, int nblk, int items) {
     const int L = (ex + 2 * G - 1) / (2 * G);
     double c = 1560.0 + L * (650.0 + 55.0 * std::min(warps, 4) + (warps > 4 ? 370.0 : 0.0));
-    if (G > 1) c += 100.0 + (ez > 4 ? 100.0 * warps * L : 0.0);
+    if (G > 1) c += 100.0 + (ez > 4 || L > 1 ? 100.0 * warps * L : 0.0);
     c += 700.0 + 320.0 * q + (q > 5 ? 2500.0 : 0.0);
     return c + (nblk > 1 ? 4500.0 + 1.6 * items : 630.0);
 }
