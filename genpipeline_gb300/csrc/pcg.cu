@@ -2212,6 +2212,26 @@ static std::vector<std::vector<int>> chip_groups(const gbsimp_ctx *ctx, const st
     return even;
 }
 
+// Whether new inner solves that the chip holds run together in persistent launches all the same. On the
+// chip large ones run one after the other, an iteration of each behind one of the last; a persistent launch
+// takes 10 us (20.7k cycles) and 25 per million elements for an iteration of all of them, fitted to 2 to
+// 8 cubes of 53 to 64 elements a side. Batches, persistent -> on chip: 57^3 x2 27.5 -> 20.9 ms, x4 43.5 -> 45,
+// x8 77.6 -> 88; 62^3 x4 49.3 -> 48.6, x8 80.6 -> 88.3; 64^3 x4 56.5 -> 52.2, x6 71.9 -> 83.4; 32^3 x24
+// 37.0 -> 28.8.
+static bool batch_streams(const gbsimp_ctx *ctx, const std::vector<ChipItem> &items,
+                          const std::vector<std::vector<int>> &groups, int per_launch) {
+    if (groups.size() < 2) return false;  // side by side on the chip
+    double chip = 0.0, elements = 0.0;
+    for (const std::vector<int> &c : groups) {
+        ChipItem ci[kChipMaxDesigns];
+        for (size_t j = 0; j < c.size(); ++j) ci[j] = items[c[j]];
+        chip += chip_cycles(ctx, ci, (int)c.size());
+    }
+    for (const ChipItem &it : items) elements += (double)it.nx * it.ny * it.nz;
+    const double launches = (double)((items.size() + per_launch - 1) / per_launch);
+    return 20700.0 * launches + 0.0518 * elements < 0.97 * chip;
+}
+
 static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int n, const gbsimp_law *glaw,
                             const gbsimp_solve_opts *o, cudaStream_t st) {
     const Law<float> law = make_law<float>(*glaw);
@@ -2305,15 +2325,23 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
             chip_try.push_back(i);
             chip_started.push_back(citem(i));
         }
+    const int per_launch = o->fused ? std::min(group, kChipMaxDesigns) : 1;
     {
-        std::vector<int> other;
+        std::vector<int> other, fit;
+        std::vector<ChipItem> fit_items;
         for (int i : fresh) {
+            const ChipItem ci = citem(i);
+            const bool on = o->max_iter > items[i].stats.iterations && chip_ok(ctx, ci);
+            (on ? fit : other).push_back(i);
+            if (on) fit_items.push_back(ci);
+        }
+        if (o->fused && fit.size() > 1 && batch_streams(ctx, fit_items, chip_groups(ctx, fit_items, per_launch), group)) {
+            other.insert(other.end(), fit.begin(), fit.end());
+            fit.clear();
+        }
+        for (int i : fit) {
             gbsimp_batch_item &it = items[i];
             ChipItem ci = citem(i);
-            if (o->max_iter <= it.stats.iterations || !chip_ok(ctx, ci)) {
-                other.push_back(i);
-                continue;
-            }
             const int64_t nd = n_dof_of(it.nx, it.ny, it.nz);
             SolveWs w = solve_ws(it.ws, it.nx, it.ny, it.nz);
             PcgWs pw = pcg_ws(w.pcg, it.nx, it.ny, it.nz);
@@ -2336,7 +2364,7 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
         }
         fresh.swap(other);
     }
-    for (const std::vector<int> &c : chip_groups(ctx, chip_started, o->fused ? std::min(group, kChipMaxDesigns) : 1)) {
+    for (const std::vector<int> &c : chip_groups(ctx, chip_started, per_launch)) {
         std::vector<ChipItem> ci;
         for (int j : c) ci.push_back(chip_started[j]);
         const int rc = chip_run(ctx, ci.data(), (int)ci.size(), budget, st);

@@ -952,24 +952,23 @@ int chip_min_blocks(const gbsimp_ctx *ctx, const ChipItem &it) {
     return chip_plans(ctx, it).least;
 }
 
-int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cudaStream_t st) {
-    if (n <= 0 || n > kChipMaxDesigns || !ctx->modal_ok || !chip_coop(ctx)) return kChipRefused;
+// The cuts of n designs of one launch and their modelled cycles; false when they do not fit together.
+static bool chip_allot(const gbsimp_ctx *ctx, const ChipItem *items, int n, ChipGeom *geo, double *cost) {
+    if (n <= 0 || n > kChipMaxDesigns || !ctx->modal_ok || !chip_coop(ctx)) return false;
     const int sms = std::min(ctx->num_sms, kChipNT);
-    ChipGeom geo[kChipMaxDesigns] = {};
     auto blocks = [&](int i) { return geo[i].Px * geo[i].Py * geo[i].Pz; };
     // CTAs: the fewest that hold each design, then more to whichever has the longest iteration,
     // up to the next number of CTAs that shortens it, while that many are left
-    double cost[kChipMaxDesigns];
     int used = 0;
     for (int i = 0; i < n; ++i) {
         const ChipPlans &P = chip_plans(ctx, items[i]);
-        if (P.least == 0) return kChipRefused;
+        if (P.least == 0) return false;
         const auto &a = P.at[n == 1 ? sms : P.least];
         geo[i] = a.g;
         cost[i] = a.cost;
         used += blocks(i);
     }
-    if (used > sms) return kChipRefused;
+    if (used > sms) return false;
     bool stuck[kChipMaxDesigns] = {};
     while (n > 1) {
         int j = -1;
@@ -988,6 +987,20 @@ int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cu
         cost[j] = P.at[c].cost;
         used += blocks(j);
     }
+    return true;
+}
+
+double chip_cycles(const gbsimp_ctx *ctx, const ChipItem *items, int n) {
+    ChipGeom geo[kChipMaxDesigns];
+    double cost[kChipMaxDesigns];
+    return chip_allot(ctx, items, n, geo, cost) ? *std::max_element(cost, cost + n) : 1e300;
+}
+
+int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cudaStream_t st) {
+    ChipGeom geo[kChipMaxDesigns] = {};
+    double cost[kChipMaxDesigns];
+    if (!chip_allot(ctx, items, n, geo, cost)) return kChipRefused;
+    auto blocks = [&](int i) { return geo[i].Px * geo[i].Py * geo[i].Pz; };
     ChipTable T;
     memset(&T, 0, sizeof T);
     T.n = n;

@@ -42,6 +42,9 @@ struct ChipItem {
 
 // Fewest CTAs that hold this solve (its grid, its packets), 0 when the chip does not. Host only.
 int chip_min_blocks(const gbsimp_ctx *ctx, const ChipItem &it);
+// Modelled SM cycles per iteration of n designs in one launch (of the slowest); 1e300 when they do not fit
+// together. Host only.
+double chip_cycles(const gbsimp_ctx *ctx, const ChipItem *items, int n);
 // Runs the inner PCGs of n designs in one cooperative launch, CTAs shared so that the designs'
 // modelled iteration times even out: at most `budget` iterations each (0: to the end). Returns
 // kChipRefused, with nothing run, when they do not fit together or the launch is refused (a context
