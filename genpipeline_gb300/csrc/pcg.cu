@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <chrono>
 #include <mutex>
+#include <new>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -1930,6 +1931,32 @@ static CsrWs csr_ws(void *ws, int64_t n) {
 
 using namespace gbs;
 
+// The entry points are C: what their containers throw ends in a status.
+template <typename F>
+static int no_throw(const char *name, F &&f) {
+    try {
+        return f();
+    } catch (const std::bad_alloc &) {
+        return set_error(GBS_ENOMEM, "%s: out of host memory", name);
+    }
+}
+
+extern "C" int gbsimp_chip_plan(int nx, int ny, int nz, int num_sms, int32_t *plan13) {
+    if (!plan13 || num_sms <= 0 || !grid_ok(nx, ny, nz)) return set_error(GBS_EINVAL, "gbsimp_chip_plan: bad arguments");
+    return no_throw("gbsimp_chip_plan", [&] {
+        memset(plan13, 0, 13 * sizeof *plan13);
+        const ChipItem it = chip_item(nx, ny, nz, pcg_ws((void *)256, nx, ny, nz), nullptr, nullptr,
+                                      apply_f64_modal_ws_bytes(nx, ny, nz));
+        ChipGeom g;
+        size_t smem;
+        if (!modal_fits(nz) || !chip_plan(nx, ny, nz, num_sms, it.xch_bytes, &g, &smem)) return (int)GBS_OK;
+        const int v[13] = {g.Px * g.Py * g.Pz, g.Px, g.Py, g.Pz, g.G, g.NYm, g.NZm, g.stride, g.q, g.items, g.multi, g.terms,
+                           (int)smem};
+        for (int i = 0; i < 13; ++i) plan13[i] = v[i];
+        return (int)GBS_OK;
+    });
+}
+
 extern "C" size_t gbsimp_pcg_ws_bytes(int nx, int ny, int nz) { return pcg_ws_bytes_impl(nx, ny, nz); }
 
 extern "C" size_t gbsimp_time_pcg_apply_ws_bytes(int nx, int ny, int nz) {
@@ -1942,9 +1969,9 @@ __global__ void fill_f32_kernel(int64_t n, float v, float *a) {
 
 __global__ void freeze_scalars_kernel(PcgScalars *sc) { sc->freeze = 1; }
 
-extern "C" int gbsimp_time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *glaw, const float *x,
-                                     const uint8_t *node_mask, int reps, void *ws, size_t ws_bytes,
-                                     double *seconds_per_launch, void *stream) {
+static int time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *glaw, const float *x,
+                          const uint8_t *node_mask, int reps, void *ws, size_t ws_bytes, double *seconds_per_launch,
+                          void *stream) {
     if (!ctx || !glaw || !x || !ws || !seconds_per_launch || reps <= 0 || reps > 100000 || !grid_ok(nx, ny, nz))
         return set_error(GBS_EINVAL, "gbsimp_time_pcg_apply: bad arguments");
     if (ws_bytes < gbsimp_time_pcg_apply_ws_bytes(nx, ny, nz))
@@ -2054,6 +2081,14 @@ extern "C" int gbsimp_time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, co
     return GBS_OK;
 }
 
+extern "C" int gbsimp_time_pcg_apply(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsimp_law *glaw, const float *x,
+                                     const uint8_t *node_mask, int reps, void *ws, size_t ws_bytes,
+                                     double *seconds_per_launch, void *stream) {
+    return no_throw("gbsimp_time_pcg_apply", [&] {
+        return time_pcg_apply(ctx, nx, ny, nz, glaw, x, node_mask, reps, ws, ws_bytes, seconds_per_launch, stream);
+    });
+}
+
 extern "C" size_t gbsimp_solve_ws_bytes(int nx, int ny, int nz) { return solve_ws_bytes_impl(nx, ny, nz); }
 
 extern "C" size_t gbsimp_pcg_csr_ws_bytes(int64_t n) { return csr_ws_bytes_impl(n); }
@@ -2069,11 +2104,14 @@ extern "C" int gbsimp_pcg_f32(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbs
     if ((uintptr_t)u & 15) return set_error(GBS_EINVAL, "gbsimp_pcg_f32: u must be 16-byte aligned");
     PcgScalars h;
     ApplyProfile prof;
-    int rc = kChipRefused;
-    for (const bool chip : {true, false})
-        if (rc == kChipRefused)
-            rc = pcg_run(ctx, nx, ny, nz, law, x, b, node_mask, u, opts->rtol, opts->max_iter, opts->check_every, ws, &h,
-                         (cudaStream_t)stream, chip, opts->profile ? &prof : nullptr, opts->fused);
+    const int rc = no_throw("gbsimp_pcg_f32", [&] {
+        int r = kChipRefused;
+        for (const bool chip : {true, false})
+            if (r == kChipRefused)
+                r = pcg_run(ctx, nx, ny, nz, law, x, b, node_mask, u, opts->rtol, opts->max_iter, opts->check_every, ws, &h,
+                            (cudaStream_t)stream, chip, opts->profile ? &prof : nullptr, opts->fused);
+        return r;
+    });
     if (rc) return rc;
     if (stats) {
         stats->apply_seconds = prof.seconds;
@@ -2104,7 +2142,9 @@ extern "C" int gbsimp_solve(gbsimp_ctx *ctx, int nx, int ny, int nz, const gbsim
     NvtxRange range("gbsimp_solve");
     if (ws_bytes < solve_ws_bytes_impl(nx, ny, nz)) return set_error(GBS_EINVAL, "gbsimp_solve: workspace too small");
     gbsimp_solve_stats s{};
-    int rc = solve_run(ctx, nx, ny, nz, law, x, f, node_mask, u, opts, &s, ws, (cudaStream_t)stream);
+    const int rc = no_throw("gbsimp_solve", [&] {
+        return solve_run(ctx, nx, ny, nz, law, x, f, node_mask, u, opts, &s, ws, (cudaStream_t)stream);
+    });
     if (rc) return rc;
     s.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (stats) *stats = s;
@@ -2541,7 +2581,7 @@ extern "C" int gbsimp_batch_round(gbsimp_ctx *ctx, gbsimp_batch_item *items, int
     NvtxRange range("gbsimp_batch_round");
     int rc = check_batch(ctx, items, n, law, opts);
     if (rc) return rc;
-    return batch_round_impl(ctx, items, n, law, opts, (cudaStream_t)stream);
+    return no_throw("gbsimp_batch_round", [&] { return batch_round_impl(ctx, items, n, law, opts, (cudaStream_t)stream); });
 }
 
 extern "C" int gbsimp_batch_solve(gbsimp_ctx *ctx, gbsimp_batch_item *items, int n, const gbsimp_law *law,
@@ -2556,7 +2596,8 @@ extern "C" int gbsimp_batch_solve(gbsimp_ctx *ctx, gbsimp_batch_item *items, int
         bool any = false;
         for (int i = 0; i < n; ++i) any = any || items[i].state == 0;
         if (!any) break;
-        rc = batch_round_impl(ctx, items, n, law, opts, (cudaStream_t)stream);
+        rc = no_throw("gbsimp_batch_solve",
+                      [&] { return batch_round_impl(ctx, items, n, law, opts, (cudaStream_t)stream); });
         if (rc) return rc;
     }
     for (int i = 0; i < n; ++i)

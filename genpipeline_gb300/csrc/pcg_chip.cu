@@ -990,6 +990,23 @@ static bool chip_allot(const gbsimp_ctx *ctx, const ChipItem *items, int n, Chip
     return true;
 }
 
+// Shared memory of a cut's largest box.
+static size_t chip_smem_of(const ChipGeom &g) {
+    const int ex = (g.nx + g.Px - 1) / g.Px, L = (ex + 2 * g.G - 1) / (2 * g.G);
+    return chip_smem(g.G * (L + 1) * g.NYm * g.NZm, L * g.G * (g.NYm - 1) * (g.NZm - 1),
+                     chip_shared(ex + 2 * g.G, g.NYm, g.NZm, g.Px, g.Py, g.Pz, true));
+}
+
+bool chip_plan(int nx, int ny, int nz, int sms, size_t xch_bytes, ChipGeom *g, size_t *smem) {
+    sms = std::min(sms, kChipNT);
+    if ((int64_t)nx * ny * nz > (int64_t)sms * 2 * kChipNT * kChipQ) return false;
+    const ChipPlans &P = chip_plans(nx, ny, nz, sms, xch_bytes);
+    if (P.least == 0) return false;
+    *g = P.at[sms].g;
+    *smem = chip_smem_of(*g);
+    return true;
+}
+
 double chip_cycles(const gbsimp_ctx *ctx, const ChipItem *items, int n) {
     ChipGeom geo[kChipMaxDesigns];
     double cost[kChipMaxDesigns];
@@ -1015,10 +1032,7 @@ int chip_run(const gbsimp_ctx *ctx, const ChipItem *items, int n, int budget, cu
         D.nblk = blocks(i);
         block0 += D.nblk;
         q = std::max(q, D.g.q);
-        const int ex = (D.g.nx + D.g.Px - 1) / D.g.Px;
-        const int L = (ex + 2 * D.g.G - 1) / (2 * D.g.G);
-        smem = std::max(smem, chip_smem(D.g.G * (L + 1) * D.g.NYm * D.g.NZm, L * D.g.G * (D.g.NYm - 1) * (D.g.NZm - 1),
-                                        chip_shared(ex + 2 * D.g.G, D.g.NYm, D.g.NZm, D.g.Px, D.g.Py, D.g.Pz, true)));
+        smem = std::max(smem, chip_smem_of(D.g));
     }
     const int v = q <= 1 ? 0 : (q <= 2 ? 1 : (q <= 4 ? 2 : (q <= 5 ? 3 : 4)));
     for (int i = 0; i < n; ++i) {

@@ -45,6 +45,9 @@ int chip_min_blocks(const gbsimp_ctx *ctx, const ChipItem &it);
 // Modelled SM cycles per iteration of n designs in one launch (of the slowest); 1e300 when they do not fit
 // together. Host only.
 double chip_cycles(const gbsimp_ctx *ctx, const ChipItem *items, int n);
+// The cut that a single design takes on a GPU of `sms` SMs, and its bytes of shared memory; false when the
+// chip does not hold the grid. Host only.
+bool chip_plan(int nx, int ny, int nz, int sms, size_t xch_bytes, ChipGeom *g, size_t *smem);
 // Runs the inner PCGs of n designs in one cooperative launch, CTAs shared so that the designs'
 // modelled iteration times even out: at most `budget` iterations each (0: to the end). Returns
 // kChipRefused, with nothing run, when they do not fit together or the launch is refused (a context

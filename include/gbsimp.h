@@ -377,6 +377,11 @@ int gbsimp_barrier_selftest(gbsimp_ctx *ctx, int extra_arrivals, double wait_sec
  * GBSIMP_DIAG_OC: 0: the OC update's cooperative launch is taken for refused. */
 enum { GBSIMP_DIAG_TIMEOUT = 1, GBSIMP_DIAG_CHIP = 2, GBSIMP_DIAG_OC = 3 };
 int gbsimp_set_diagnostic(gbsimp_ctx *ctx, int key, int64_t value);
+/* How the on-chip PCG of gbsimp_solve cuts a grid on a GPU of num_sms SMs (host only, for tests): plan =
+ * {blocks (0: the chip does not hold the grid), cuts along x, y, z, pairs of x slabs per block, node strides
+ * of a row's plane along y and z, nodes of the largest block, places per thread, room for packets to
+ * wait for, for nodes of several neighbours and for the terms of their sums, bytes of shared memory}. */
+int gbsimp_chip_plan(int nx, int ny, int nz, int num_sms, int32_t *plan13);
 
 /* ---- reductions used by the host loops -------------------------------------------- */
 /* out (device double) = sum_i a_i * b_i over n FP64 entries, fixed block order. */
