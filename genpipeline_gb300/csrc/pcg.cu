@@ -2257,7 +2257,8 @@ static std::vector<std::vector<int>> chip_groups(const gbsimp_ctx *ctx, const st
 // takes 10 us (20.7k cycles) and 25 per million elements for an iteration of all of them, fitted to 2 to
 // 8 cubes of 53 to 64 elements a side. Batches, persistent -> on chip: 57^3 x2 27.5 -> 20.9 ms, x4 43.5 -> 45,
 // x8 77.6 -> 88; 62^3 x4 49.3 -> 48.6, x8 80.6 -> 88.3; 64^3 x4 56.5 -> 52.2, x6 71.9 -> 83.4; 32^3 x24
-// 37.0 -> 28.8.
+// 37.0 -> 28.8. Whole inner solves only: in rounds of a budget designs come and go one by one, and a
+// stream of 24 to 96 cubed served 39.9 solves/s with all that fit on the chip, 38.0 by this rule.
 static bool batch_streams(const gbsimp_ctx *ctx, const std::vector<ChipItem> &items,
                           const std::vector<std::vector<int>> &groups, int per_launch) {
     if (groups.size() < 2) return false;  // side by side on the chip
@@ -2375,7 +2376,8 @@ static int batch_round_impl(const gbsimp_ctx *ctx, gbsimp_batch_item *items, int
             (on ? fit : other).push_back(i);
             if (on) fit_items.push_back(ci);
         }
-        if (o->fused && fit.size() > 1 && batch_streams(ctx, fit_items, chip_groups(ctx, fit_items, per_launch), group)) {
+        if (o->fused && budget == 0 && fit.size() > 1 &&
+            batch_streams(ctx, fit_items, chip_groups(ctx, fit_items, per_launch), group)) {
             other.insert(other.end(), fit.begin(), fit.end());
             fit.clear();
         }

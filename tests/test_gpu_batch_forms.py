@@ -2,6 +2,7 @@
 the chip would hold them one after the other for longer; the displacements meet the tolerance in both."""
 import numpy as np
 import pytest
+import torch
 
 from genpipeline_gb300 import _lib as L
 from genpipeline_gb300 import bcs
@@ -10,7 +11,8 @@ from genpipeline_gb300.engine import n_elem
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
-PERSISTENT, GRAPH, CHIP = 1, 2, 3  # stats.inner_active of a paused solve
+KERNEL = {"chip": "pcg_chip_kernel", "persistent": "pcg_fused_kernel", "graph": "apply_modal_kernel"}
+PAUSED = {1: "persistent", 2: "graph", 3: "chip"}  # stats.inner_active
 
 
 def _designs(sizes):
@@ -22,21 +24,52 @@ def _designs(sizes):
     return out
 
 
-@pytest.mark.parametrize("sizes,fused,form", [((57,) * 2, True, CHIP), ((57,) * 5, True, PERSISTENT),
-                                              ((57,) * 5, False, CHIP), ((64,) * 4, True, CHIP),
-                                              ((64,) * 6, True, PERSISTENT), ((32,) * 20, True, CHIP),
-                                              ((8,) * 30, True, CHIP), ((67, 67), True, PERSISTENT),
-                                              ((67, 67), False, GRAPH)])
-def test_form_and_residual(sizes, fused, form):
+def _kernels(run):
+    """The names of the kernels that run() launches."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        run()
+        torch.cuda.synchronize()
+    return {e.name for e in prof.events()}
+
+
+@pytest.fixture(scope="module", autouse=True)
+def tracing():
+    """A process's first profile may come back empty."""
+    for _ in range(5):
+        if _kernels(lambda: torch.zeros(1 << 20, device="cuda").add_(1)):
+            return
+    pytest.skip("no kernel names from the profiler here")
+
+
+@pytest.mark.parametrize("sizes,fused,form,paused", [
+    ((57,) * 2, True, "chip", "chip"), ((57,) * 5, True, "persistent", "chip"), ((57,) * 5, False, "chip", "chip"),
+    ((64,) * 4, True, "chip", "chip"), ((64,) * 6, True, "persistent", "chip"), ((32,) * 20, True, "chip", "chip"),
+    ((8,) * 30, True, "chip", "chip"), ((67, 67), True, "persistent", "persistent"), ((67, 67), False, "graph", "graph")])
+def test_form_and_residual(sizes, fused, form, paused):
+    # rounds of whole inner solves
+    designs = _designs(sizes)
+    b = BatchFEM(fused=fused)
+    for d in designs:
+        b.add(d)
+    names = _kernels(b.round)
+    assert {f for f, k in KERNEL.items() if any(k in n for n in names)} == {form}
+    while b.items:
+        b.round()
+    _check(designs)
+    # rounds of a budget
     designs = _designs(sizes)
     b = BatchFEM(fused=fused, round_iters=24)
     for d in designs:
         b.add(d)
     b.round()
-    assert {d._item.stats.inner_active for d in designs} == {form}
+    assert {PAUSED[d._item.stats.inner_active] for d in designs} == {paused}
     b.opts.check_every = 0
     while b.items:
         b.round()
+    _check(designs)
+
+
+def _check(designs):
     for d in designs[:3]:
         assert d.stats["status"] == L.GBS_OK and d.stats["relres"] <= 1e-8, d.stats
         dof = bcs.dof_mask(*d.grid, d.fixed_dofs)
