@@ -19,6 +19,7 @@ workload.
 from __future__ import annotations
 
 import argparse
+import ctypes
 import json
 import os
 import re
@@ -201,6 +202,18 @@ def _measured_peak():
         return 6800.0, "fallback"
 
 
+def _on_chip(grid, dev):
+    """Whether a solve of this grid runs in the on-chip form on this GPU."""
+    import torch
+
+    from genpipeline_gb300 import _lib as L
+
+    plan = (ctypes.c_int32 * 13)()
+    L.check(L.load().gbsimp_chip_plan(*(int(n) for n in grid), torch.cuda.get_device_properties(dev).multi_processor_count,
+                                      plan))
+    return plan[0] > 0
+
+
 def _profiled_traffic(workload="simp64"):
     """DRAM bytes per launch of the one-kernel PCG iteration from the committed ncu summary of the
     workload."""
@@ -235,11 +248,11 @@ def batch_designs():
 
 
 def measure_batch(repeats=2):
-    """FEM solves/s of the 8-design batch: plain = one solve per design (graph-loop PCG, one
-    design on the GPU at a time); served = the designs together in gbsimp_batch_round with the
+    """FEM solves/s of the 8-design batch: plain = one solve per design (one design on the GPU at a
+    time); served = the designs together in gbsimp_batch_round with the
     configuration the autotuner chose for this grid class (timed once per candidate during the
-    warm-up, then cached); served_rule = the untuned default (one persistent launch, SMs in
-    proportion to element counts). Cold starts (u0 = 0) everywhere."""
+    warm-up, then cached); served_rule = the untuned default (as many designs per launch as
+    are resident together). Cold starts (u0 = 0) everywhere."""
     import torch
 
     from genpipeline_gb300 import autotune as A
@@ -782,9 +795,7 @@ def run_ours(a):
         # out; x read and written every other iteration (two-step update): 10 words per DOF
         # on average, the basis of one standard Jacobi-PCG iteration
         alg_bytes = 4 * (10 * nd + ne)
-        # (a grid that the chip holds moves none of them: frac then says how much faster than a pass
-        # over memory the iteration is)
-        kname = "one single-reduction PCG iteration: s, r, u, w = DKDu, p, x (pcg_chip_kernel, or apply_modal_kernel)"
+        kname = "apply_modal_kernel (one single-reduction PCG iteration: s, r, u, w = DKDu, p, x)"
     else:
         alg_bytes = 4 * (7 * nd + ne)  # r, dinv, p_old, x_u, x in; p_new, Ap, x_u out
         kname = "apply_tile_kernel<PCG> (K(x)p fused with p = z + beta p, x update, p.Ap)"
@@ -795,6 +806,13 @@ def run_ours(a):
             "traffic": _profiled_traffic(a.workload), "alg_bytes_per_launch": alg_bytes, "launch_us": per_launch * 1e6,
             "fp32_flops_per_launch_dense_equiv": 1152 * ne,
             "est_share_of_step": pcg_iters * per_launch / t}
+    if path == "modal" and _on_chip(GRID, dev):
+        # every vector stays in registers and shared memory: no bytes to hold against the memory's rate
+        roof.update(bound="latency", kernel="pcg_chip_kernel (all iterations of an inner PCG in one launch; per iteration)",
+                    achieved=None, peak=None, peak_source=None, unit=None, frac=None, alg_bytes_per_launch=0,
+                    streaming_equivalent_GBs=achieved,
+                    note="launch_us: 50 iterations and the launch's loads and stores, per iteration; "
+                         "streaming_equivalent_GBs: what a pass over memory would have to move")
 
     # ---- CPU baseline: the oracle on the same trajectory, from the GPU's state ----------
     cpu = None

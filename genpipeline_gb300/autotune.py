@@ -4,9 +4,11 @@ A batch of designs solved together (``BatchFEM.solve_all``: the 8-design evaluat
 ``VoxelFEMEvaluator.evaluate_batch``, ``BatchSIMP``'s rounds) has three free parameters that
 the library exposes through ``gbsimp_solve_opts``:
 
-- the form: designs sharing persistent cooperative launches (``fused`` = 1) or each design in
-  its own device-driven graph loop (``fused`` = 0);
-- the SM share of each design in a persistent launch (``batch_share``): in proportion to its
+- the form: designs sharing cooperative launches (``fused`` = 1: on the chip the grids that it
+  holds, in the persistent kernel the others) or one design at a time (``fused`` = 0: a launch each on the
+  chip, a device-driven graph loop for the others);
+- the SM share of each design in a persistent launch (``batch_share``; on the chip the shares follow its
+  cost model): in proportion to its
   element count, or to element count x longest extent (Jacobi-PCG iteration counts grow about
   with the longest extent, so the designs of a launch then finish together instead of small
   ones leaving their SMs idle while a large one converges);
@@ -36,16 +38,16 @@ from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 @dataclass(frozen=True)
 class BatchConfig:
-    fused: int = 1        # 1: persistent launches shared by designs; 0: one graph loop per design
+    fused: int = 1        # 1: launches shared by designs; 0: one design at a time
     batch_share: int = 0  # 0: SMs by element count; 1: by element count x longest extent
-    batch_group: int = 0  # designs per persistent launch (0: as many as are resident together)
+    batch_group: int = 0  # designs per launch (0: as many as are resident together)
 
     def label(self) -> str:
         if not self.fused:
-            return "graph loop per design"
+            return "one design at a time (on the chip, or its graph loop)"
         share = "elements" if self.batch_share == 0 else "elements x extent"
         group = "all resident" if self.batch_group == 0 else f"<= {self.batch_group}"
-        return f"persistent, share by {share}, {group} per launch"
+        return f"shared launches (on the chip, or persistent by {share}), {group} per launch"
 
 
 CANDIDATES: Tuple[BatchConfig, ...] = (

@@ -3,9 +3,10 @@
 The reference evaluates designs one at a time: ``VoxelFEMEvaluator.evaluate_batch`` fans
 ``GPUVoxelFEM.solve`` calls out to a thread pool, and each call assembles its own CSR
 matrix and runs its own PCG loop (voxel_fem.py:559-611, gpu_fem_solver.py:76-133). Here a
-batch shares the GPU inside one persistent kernel per round. Every design gets a share of
-the SMs, its own grid barrier and its own scalars; the FP64 defect correction runs in
-lockstep rounds around those launches.
+batch shares the GPU inside one cooperative kernel per round: on the chip the designs whose grids it
+holds, in a persistent streaming kernel the larger ones. Every design gets a share of
+the SMs and its own scalars; the FP64 defect correction runs in lockstep rounds around those
+launches.
 """
 from __future__ import annotations
 
@@ -180,8 +181,7 @@ class BatchFEM:
 
 class SolveQueue:
     """The native solve queue (gbsimp_queue_*): designs are submitted at any time, each poll
-    runs one defect-correction round for everything queued (the persistent batched PCG
-    inside) and hands back the designs that finished. The same continuous batching as
+    runs one defect-correction round for everything queued (the batched PCG inside) and hands back the designs that finished. The same continuous batching as
     BatchFEM, with the queue kept by the library."""
 
     def __init__(self, engine: Optional[Engine] = None, law: Optional[L.Law] = None, rtol: float = 1e-8,
@@ -236,7 +236,7 @@ class SolveQueue:
 
 def solve_plain(designs: List[FEMDesign], engine: Optional[Engine] = None, law: Optional[L.Law] = None,
                 rtol: float = 1e-8, inner_rtol: float = INNER_RTOL) -> List[FEMDesign]:
-    """The one-design-at-a-time form: one gbsimp_solve (graph-loop PCG) per design."""
+    """The one-design-at-a-time form: one gbsimp_solve per design."""
     eng = engine or get_engine()
     law = law or L.make_law("modified", 3.0)
     bf = BatchFEM(eng, law)

@@ -83,10 +83,10 @@ __global__ void __launch_bounds__(kEdofNT) apply_edof_kernel(int64_t n_elem, int
 }
 
 // The energy's 24 products, exact to their rounding errors, are summed in FP32 pairs (2^-46); an FP64 sum,
-// with its conversions, took half of the kernel's 16 us at 65536 elements (6.1 so). The displacements are
+// with its conversions, took half of the kernel's 16 us at 65536 elements (6.4 so). The displacements are
 // scaled by a power of two to a largest component between 1 and 2, so that displacements of any size keep
-// to the pairs (at 1e-13 and below the sums ran in FP64 and the kernel took 10.7 us). Where a pair does not hold the
-// sum all the same (infinities, NaN, a stiffness near either end of the range) it runs in FP64.
+// to the pairs (a call took 17 to 18 us at every size; unscaled, 15 to 19, and 23 at 1e-13 and below, where
+// the sums ran in FP64). Where a pair does not hold the sum all the same (infinities, NaN, a stiffness near either end of the range) it runs in FP64.
 template <typename I>
 __global__ void __launch_bounds__(kEdofNT) sens_edof_kernel(int64_t n_elem, int64_t n_dof, const void *edof,
                                                             Law<float> law, const KeF ke, const float *x,

@@ -1121,9 +1121,10 @@ struct EventPair {
 };
 
 // ---- the on-chip form (pcg_chip.cu) ---------------------------------------------------------
-// Whenever the grid fits the chip: it is the faster form at every size that does. us per iteration of
-// a solve, streaming in the graph loop -> on the chip: 8x4x4 7.5 -> 1.7, 32x8x8 7.9 -> 3.9, 32^3
-// 8.4 -> 4.2, 48^3 10.7 -> 5.3, 95x47x33 11.9 -> 6.7, 64^3 (about the most it holds) 13.9 -> 8.9.
+// Whenever the grid fits the chip: it is the faster form of a single solve at every size that does. us per
+// iteration of a solve, streaming in the graph loop -> on the chip: 8x4x4 8.3 -> 1.9, 32x8x8 8.0 -> 3.7,
+// 33^3 8.4 -> 4.8, 50^3 11.0 -> 6.3, 300x1x300 26 -> 6.1, 20x20x400 52 -> 6.6, 64^3 14.0 -> 8.7, 66^3 (the
+// largest cube it holds) 14.3 -> 10.1.
 static inline bool chip_ok(const gbsimp_ctx *ctx, const ChipItem &it) {
     return use_modal(ctx, it.nz) && chip_min_blocks(ctx, it) > 0;
 }

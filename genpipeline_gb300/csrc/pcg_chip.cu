@@ -8,7 +8,8 @@
 // the partial sums and the launch gap, where its arithmetic takes 1.4 us of the SMs' FP32 rate.
 // 152 SMs hold 34 MB of shared memory and 39 MB of registers; the PCG state of 64^3 is 20 MB.
 // Here an iteration of 32^3 takes 4.1 us (streaming 8.4): march 1.4, exchange 2.2, sums 0.3,
-// update 0.2; one of 64^3 8.9, of which 0.8 is its kernel's code not fitting the instruction cache.
+// update 0.2; one of 64^3 8.8, of which 0.8 is its kernel's code not fitting the instruction cache
+// (launches of 2000 iterations; with the loads and stores of one of 50 9.8 to 10.0 at 64^3).
 // Split. The elements are cut into Px x Py x Pz boxes, one per CTA. A CTA holds all nodes of its
 // box, so nodes on a face between boxes are held by both. The box's K u is a partial sum there;
 // per iteration the CTAs exchange those partials (a node's 12 bytes) and three sums, and every

@@ -13,7 +13,7 @@ parameter set, in order; a sentinel result with ``success=False`` when ``latent_
 missing; ``OptimizationSample`` records in ``evaluation_history``), but replaces the thread
 pool of one-solve-per-design calls (:559-611) with one batched pipeline: all latents are
 decoded in one call, all grids are prepared in one launch sequence, and all solves share the
-persistent batched PCG (``BatchFEM``: rounds of gbsimp_batch_round with continuous batching).
+batched PCG (``BatchFEM``: rounds of gbsimp_batch_round with continuous batching).
 
 The solve runs to rtol 1e-8 (FP32 PCG with FP64 defect correction) instead of the reference
 path's 1e-3 / 200 iterations, so the outputs are those of the exact discrete solution.

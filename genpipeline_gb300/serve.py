@@ -13,7 +13,7 @@ milliseconds whatever the grid sizes. Between two rounds the server:
 - retires the designs that finished in the round.
 
 So a request that arrives while others are on the GPU joins within one round, and its work
-overlaps theirs inside the same persistent launch (``gbsimp_batch_round``). A finished
+overlaps theirs inside the same round's launches (``gbsimp_batch_round``). A finished
 request's displacement stays on the device in a warm-start cache keyed by (n, seed, load),
 so a repeated design starts from its previous solution. Refused and cancelled requests get the
 reference's failure record: every output FEM_SENTINEL and a ``failure_reason``

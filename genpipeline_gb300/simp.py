@@ -38,7 +38,7 @@ class SolveSpec:
     inner_rtol: float = INNER_RTOL  # FP32 PCG reduction per outer correction (engine.INNER_RTOL)
     max_iter: int = 200000
     max_outer: int = 30
-    fused: bool = False         # persistent one-launch PCG (grid barriers) instead of the graph loop
+    fused: bool = False         # grids past the chip: persistent one-launch PCG instead of the graph loop
     # warm start of solve k >= 3: u_{k-1} + warm_theta (u_{k-1} - u_{k-2}) (0: u_{k-1}); the value
     # of the native loop (gbsimp_simp_run), whose designs this loop reproduces bit for bit
     warm_theta: float = 0.5

@@ -7,8 +7,8 @@ DOFs to 1e-10, as the reference solves those directly), the floored law
 ``max(x, 1e-3)^penal``, the filtered sensitivity, the GPU OC variant, then a fresh compliance
 solve (1e-6 / 2000) whose displacement warm-starts the next iteration, and the early stop
 after three changes of compliance below 1%. The solves of all problems still running go
-through ``BatchFEM`` rounds together (one persistent launch per round, up to 24 designs per
-launch, each on its own share of the SMs). The sensitivity, filter and OC steps are launched
+through ``BatchFEM`` rounds together (up to 16 designs per launch on the chip, up to 24 of
+larger grids per persistent launch, each on its own share of the SMs). The sensitivity, filter and OC steps are launched
 per problem on the same stream. ``bc_fn(nx, ny, nz, bcs, force)`` gives each problem's load
 and clamped DOFs (default: ``SIMPSolverGPU._get_bcs``).
 """

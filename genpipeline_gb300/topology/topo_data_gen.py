@@ -11,7 +11,7 @@ mass, parameters; :246-289).
 
 Changed: instead of one solver per sample in a thread pool (:291-307), ``generate`` draws a
 batch of samples and runs them together through ``BatchSIMP``. Every SIMP iteration's FEM
-solves of all samples share persistent batched launches, so many small grids of uneven sizes
+solves of all samples share batched launches, so many small grids of uneven sizes
 fill the GPU. The iteration follows ``SIMPSolverGPU.run``. Each sample gets its ``GEOM_BCS``
 entry (which the reference's GPU branch drops: its ``DenseGPUSolver`` takes no boundary
 conditions, :208-224) through ``bcs.generator``: the clamped faces and loads of the CPU

@@ -80,15 +80,18 @@ typedef struct gbsimp_solve_opts {
                              graph-loop trips of 12 there), after which the round returns and the
                              paused solves resume in the next one; 0 = every inner PCG runs to
                              its tolerance within the round */
-    int32_t fused;        /* grids that the chip does not hold: 1 = persistent fused PCG kernel, 0 = graph
-                             loop, one launch per iteration */
-    int32_t profile;      /* 1 = time every PCG apply launch with CUDA events (stats) */
-    int32_t batch_share;  /* batched persistent launches: how the SMs are shared among the designs
+    int32_t fused;        /* a grid that the chip does not hold: 1 = persistent fused PCG kernel, 0 = graph
+                             loop, one launch per iteration. One that it holds runs there, a design per
+                             launch in batches with 0; with 1 a batch's designs share launches, on the
+                             chip or in the persistent kernel */
+    int32_t profile;      /* 1 = time every PCG apply launch with CUDA events (stats); on the chip its one
+                             launch, counted as its iterations */
+    int32_t batch_share;  /* batched persistent launches (on the chip its cost model): how the SMs are shared among the designs
                              of one launch. 0 = in proportion to element counts; 1 = in proportion
                              to element counts x longest grid extent (Jacobi-PCG iteration counts
                              grow about with it, so the designs of a launch finish together) */
-    int32_t batch_group;  /* batched persistent launches: at most this many designs per launch
-                             (0 or more than 24: 24) */
+    int32_t batch_group;  /* batched launches: at most this many designs per launch (0 or more than 24:
+                             24; on the chip at most 16) */
     int32_t residual_fp64; /* 1 = the outer residual's element products in FP64 at every rtol;
                               0 = in double-float for rtol >= 1e-9 (see gbsimp_solve) */
 } gbsimp_solve_opts;
@@ -276,7 +279,9 @@ typedef struct gbsimp_batch_item {
 
 /* One round of the FP64 defect correction for every active item: FP64 residuals (one sync
  * for all), then the FP32 PCG of every item still above rtol, then the FP64 corrections.
- * Items whose grids the chip holds run there, up to 16 designs per launch with opts->fused.
+ * Items whose grids the chip holds run there, up to 16 designs per launch with opts->fused, unless
+ * they would run one after the other there for longer than together in persistent launches (five cubes of 57,
+ * say; fused rounds without a budget only) or the launch is refused.
  * Of the others, with opts->fused the PCGs run as cooperative launches of a persistent kernel, up to 24
  * items per launch (packed greedily from the items that are resident together), each item on
  * its own share of the SMs with its own grid barrier and scalars, converging independently.
