@@ -468,7 +468,8 @@ static FilterTile filter_tile(const gbsimp_ctx *ctx, int nx, int ny, int nz, int
 // taps (rmin up to sqrt 2) 48^3 3.7 -> 5.2 us, 256x256x100 67 -> 81; 19 taps 32^3 5.0 -> 6.2, 33^3
 // 6.4 -> 5.8, 32x8x8 6.6 -> 5.4 but 3x60x60 5.1 -> 6.6; 81 taps 32^3 13.6 -> 12.0, 1x64x64 7.8 -> 9.5,
 // 1x450x450 20.5 -> 13.0, 1x1x200000 17 -> 164 (the columns beyond the grid are all zeros); 93 taps
-// 450x450x1 27 -> 34 (three of a thread's four elements lie outside); 895 taps 1x450x450 174 -> 203.
+// 450x450x1 27 -> 34 (three of a thread's four elements lie outside); 485 taps
+// 1x450x450 98 -> 61, 739 taps 146 -> 170.
 // With the sums of weights to form as well (own), which the tile does one after the other: 81 taps 32^3
 // 13.5 -> 17.7, 33^3 21.0 -> 16.0, 19 taps 64^3 9.4 -> 8.9, 256x256x100 142 -> 153, 895 taps 2x300x300
 // 171 -> 207.
@@ -476,7 +477,7 @@ static bool filter_tiled(int nx, int ny, int nz, int taps, bool own) {
     const int64_t n = (int64_t)nx * ny * nz;
     const int lo = std::min(nx, std::min(ny, nz)), hi = std::max(nx, std::max(ny, nz));
     if (taps <= 7) return false;
-    if (lo == 1) return !own && taps >= 60 && taps < 800 && n >= 100000 && n / hi >= 32 && nz >= 32;
+    if (lo == 1) return !own && taps >= 60 && taps < 600 && n >= 100000 && n / hi >= 32 && nz >= 32;
     if (own) return taps >= 60 && n > 33000 && lo > 2;
     return taps >= 60 || n > 33000 || (nz < 16 && lo > 3);
 }
@@ -501,9 +502,9 @@ int filter_launch(const gbsimp_ctx *ctx, int nx, int ny, int nz, double rmin, in
     const unsigned blocks = (unsigned)(((nx + T.ti - 1) / T.ti) * T.nbj * T.nbk);
     const size_t smem = sizeof(float) * (size_t)(T.ti + 2 * R) * (T.tj + 2 * R) * ((4 * T.kt + 2 * R + 3) & ~3);
     static void (*const kern[])(int, int, int, FilterTile, FilterCols, int, const float *, const float *,
-                                const uint8_t *, float *) = {filter_kernel<0>, filter_kernel<1>, filter_kernel<2>,
-                                                             filter_kernel<3>, filter_kernel<4>, filter_kernel<5>};
-    kern[R]<<<blocks, nt, smem, st>>>(nx, ny, nz, T, F, mode, hs, in, preserved, out);
+                                const uint8_t *, float *) = {filter_kernel<1>, filter_kernel<2>, filter_kernel<3>,
+                                                             filter_kernel<4>, filter_kernel<5>};
+    kern[R - 1]<<<blocks, nt, smem, st>>>(nx, ny, nz, T, F, mode, hs, in, preserved, out);
     GBS_LAUNCH_CHECK("filter_kernel");
     return GBS_OK;
 }

@@ -30,7 +30,7 @@ def test_filter_against_oracle(grid, rmin):
 
 @pytest.mark.parametrize("grid,rmin", [((48, 30, 33), 1.4), ((48, 30, 33), 1.5), ((32, 32, 32), 1.5), ((33, 33, 33), 1.5),
                                        ((32, 32, 32), 2.5), ((33, 33, 33), 2.5), ((4, 60, 15), 2.0), ((4, 60, 16), 2.0),
-                                       ((1, 31, 3300), 2.5), ((1, 32, 3300), 2.5), ((1, 320, 320), 6.0),
+                                       ((1, 31, 3300), 2.5), ((1, 32, 3300), 2.5), ((1, 320, 320), 5.0), ((1, 320, 320), 5.5), ((1, 320, 320), 6.0),
                                        ((3300, 32, 1), 3.0), ((1, 1, 3000), 4.0), ((3000, 1, 1), 1.5)])
 def test_both_forms_at_the_lines_between_them(grid, rmin):
     """Either side of each line of the choice between a tap at a time and tiles."""
